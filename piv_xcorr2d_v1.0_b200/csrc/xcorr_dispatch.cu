@@ -27,7 +27,6 @@ cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t 
     X(24, 24, 4, 96) \
     X(24, 24, 8, 192) \
     X(24, 24, 2, 64) \
-    X(32, 32, 8, 128) \
     X(32, 32, 4, 128) \
     X(32, 32, 2, 64) \
     X(32, 32, 8, 256) \
@@ -46,8 +45,8 @@ cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t 
     X(48, 24, 8, 192) \
     X(24, 48, 4, 96) \
     X(24, 48, 2, 64) \
-    X(24, 48, 4, 64) \
-    X(24, 48, 8, 96) \
+    X(24, 48, 4, 128) \
+    X(24, 48, 8, 192) \
     X(32, 16, 8, 128) \
     X(32, 16, 4, 64) \
     X(32, 16, 8, 256) \
@@ -70,6 +69,11 @@ template <int WSX, int WSY, int NT>
 cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, int K, cudaStream_t s);
 extern template cudaError_t launch_shape_block<32, 32, 128>(const XcorrArgs &, bool, int, cudaStream_t);
 
+// the warp form (a window pair per warp, four warps per CTA), listed before them
+template <int NW>
+cudaError_t launch_pair(const XcorrArgs &a, bool deformed, int K, cudaStream_t s);
+extern template cudaError_t launch_pair<4>(const XcorrArgs &, bool, int, cudaStream_t);
+
 // Variants of the persistent batch launch (two per shape; the batch autotuner picks one
 // per shape group).
 template <int WSX, int WSY, int B, int NT>
@@ -84,7 +88,6 @@ cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaSt
     X(24, 24, 8, 96) \
     X(24, 24, 4, 96) \
     X(32, 32, 4, 128) \
-    X(32, 32, 8, 128) \
     X(48, 48, 4, 96) \
     X(48, 48, 2, 96) \
     X(64, 64, 2, 128) \
@@ -111,6 +114,7 @@ struct Variant {
     cudaError_t (*fn)(const XcorrArgs &, bool, int, cudaStream_t);
 };
 const Variant kVariants[] = {
+    {32, 32, 8, 128, &launch_pair<4>},
 #define PIV_X(WX, WY, B, NT) {WX, WY, B, NT, &launch_shape<WX, WY, B, NT>},
     PIV_XCORR_VARIANTS(PIV_X)
 #undef PIV_X
@@ -148,12 +152,17 @@ bool xcorr_variant_shape(int wsx, int wsy, int variant, int *B, int *NT)
     return true;
 }
 
+template <int NW>
+cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, int K, cudaStream_t s);
+extern template cudaError_t launch_pair_batch<4>(const XcorrBatch &, bool, int, cudaStream_t);
+
 namespace {
 struct BatchVariant {
     int wsx, wsy, B, NT;
     cudaError_t (*fn)(const XcorrBatch &, bool, int, cudaStream_t);
 };
 const BatchVariant kBatchVariants[] = {
+    {32, 32, 8, 128, &launch_pair_batch<4>},
 #define PIV_X(WX, WY, B, NT) {WX, WY, B, NT, &launch_shape_batch<WX, WY, B, NT>},
     PIV_XCORR_BATCH_VARIANTS(PIV_X)
 #undef PIV_X

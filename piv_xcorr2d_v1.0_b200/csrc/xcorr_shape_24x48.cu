@@ -5,8 +5,8 @@
 namespace piv {
 template cudaError_t launch_shape<24, 48, 4, 96>(const XcorrArgs &, bool, int, cudaStream_t);
 template cudaError_t launch_shape<24, 48, 2, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 48, 4, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 48, 8, 96>(const XcorrArgs &, bool, int, cudaStream_t);
+template cudaError_t launch_shape<24, 48, 4, 128>(const XcorrArgs &, bool, int, cudaStream_t);
+template cudaError_t launch_shape<24, 48, 8, 192>(const XcorrArgs &, bool, int, cudaStream_t);
 template cudaError_t launch_shape_batch<24, 48, 4, 96>(const XcorrBatch &, bool, int, cudaStream_t);
 template cudaError_t launch_shape_batch<24, 48, 2, 64>(const XcorrBatch &, bool, int, cudaStream_t);
 }

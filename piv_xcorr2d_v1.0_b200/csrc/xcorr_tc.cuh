@@ -43,6 +43,68 @@
 
 namespace piv {
 
+// Byte b of w as a float: the byte is placed into the low mantissa bits of 2^23
+// (0x4B0000bb), then 2^23 is subtracted -- exact for 0..255, one PRMT + one FADD.
+template <int b>
+__device__ __forceinline__ float byte_to_float(uint32_t w)
+{
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | b)) - 8388608.0f;
+}
+
+template <int WSX>
+__device__ __forceinline__ void load_u8_row(const uint8_t *p, float (&v)[WSX])
+{
+    uintptr_t ad = reinterpret_cast<uintptr_t>(p);
+    if constexpr (WSX % 8 == 0) {
+        if ((ad & 7) == 0) {
+#pragma unroll
+            for (int q = 0; q < WSX / 8; ++q) {
+                uint2 u = __ldg(reinterpret_cast<const uint2 *>(p) + q);
+                v[8 * q + 0] = byte_to_float<0>(u.x);
+                v[8 * q + 1] = byte_to_float<1>(u.x);
+                v[8 * q + 2] = byte_to_float<2>(u.x);
+                v[8 * q + 3] = byte_to_float<3>(u.x);
+                v[8 * q + 4] = byte_to_float<0>(u.y);
+                v[8 * q + 5] = byte_to_float<1>(u.y);
+                v[8 * q + 6] = byte_to_float<2>(u.y);
+                v[8 * q + 7] = byte_to_float<3>(u.y);
+            }
+            return;
+        }
+    }
+    if ((ad & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < WSX / 4; ++q) {
+            uint32_t u = __ldg(reinterpret_cast<const uint32_t *>(p) + q);
+            v[4 * q + 0] = byte_to_float<0>(u);
+            v[4 * q + 1] = byte_to_float<1>(u);
+            v[4 * q + 2] = byte_to_float<2>(u);
+            v[4 * q + 3] = byte_to_float<3>(u);
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < WSX; ++i) v[i] = (float)__ldg(p + i);
+}
+
+template <int WSX>
+__device__ __forceinline__ void load_f32_row(const float *p, float (&v)[WSX])
+{
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+#pragma unroll
+        for (int q = 0; q < WSX / 4; ++q) {
+            float4 u = __ldg(reinterpret_cast<const float4 *>(p) + q);
+            v[4 * q] = u.x;
+            v[4 * q + 1] = u.y;
+            v[4 * q + 2] = u.z;
+            v[4 * q + 3] = u.w;
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < WSX; ++i) v[i] = __ldg(p + i);
+}
+
 template <int WS>
 struct TwTable {
     float c[WS], s[WS];
