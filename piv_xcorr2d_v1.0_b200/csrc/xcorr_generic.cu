@@ -20,21 +20,31 @@
 //   inverse  in-place decimation-in-frequency stages (natural input, digit-reversed output,
 //            the same permutation), then |.|/N in place;
 //   peaks    the fftshifted plane is read through index maps: 4-neighbour local maxima
-//            inside the search region, their count, Npeak_save rounds of a block arg-max
-//            (value desc, then lower index), the 3-point Gaussian fit with the FP64
-//            log-ratio denominator, predictor, limits, NaN/Inf removal.
+//            inside the search region, their count, one scan with a top-list per thread (up to
+//            8 saved peaks) or Npeak_save rounds of a block arg-max (more), value desc, then
+//            lower index; the 3-point Gaussian fit with the FP64 log-ratio denominator,
+//            predictor, limits, NaN/Inf removal.
+// What bounds it: shared-memory passes and their index arithmetic.  All index maps are tables
+// or multiply-high divisions by per-stage constants, and the peaks are found in one scan: a runtime
+// division or remainder per point and stage and a scan per saved peak took 0.946 ms for the 7,676
+// 40x40 windows and 0.892 ms for the 1,333 96x96 windows of a 2048x1536 frame at 50 % overlap,
+// now 0.394 and 0.293 ms.
 // Twiddles are exp(-2 pi i t/N) tables computed per CTA in FP64 and rounded once to FP32.
 #include <cfloat>
 #include <climits>
 
 #include "piv_common.cuh"
+#include "xcorr_kernel.cuh"
 
 namespace piv {
 
-// Radices of the two dimensions (outermost first) and where the plane lives.
+// Radices of the two dimensions (outermost first) and where the plane lives; the constants of
+// the index divisions (div_by): mx[s], my[s] by M of stage s (the product of the radices after
+// it), px[s], py[s] by the butterflies per line N / radix, dx by ws_x.
 struct GenericPlan {
     int nfx, nfy;
     int fx[12], fy[12];
+    uint32_t mx[12], my[12], px[12], py[12], dx;
     int in_smem;  // 1: the plane in shared memory, 0: in the CTA's workspace slab
     int any;      // a radix above 7 (prime up to 251): the local-array stage
 };
@@ -42,23 +52,34 @@ struct GenericPlan {
 namespace {
 
 constexpr int kGenThreads = kGenericThreads;
+constexpr int kGenWarps = kGenThreads / 32;
 constexpr int kGenSmemPlane = 20480;  // complex points of a plane kept in shared memory
 
-__device__ __forceinline__ float2 gmul(float2 a, float2 b)
+// n / d by a multiply-high with ceil(2^32 / d) (0 for d = 1): exact while n * d < 2^32, and the
+// kernel's n stay below 2^20 points with d up to 1024.
+__host__ __device__ inline uint32_t div_magic32(int d)
 {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return d > 1 ? (uint32_t)((0x100000000ull + (uint64_t)d - 1) / (uint64_t)d) : 0u;
+}
+__device__ __forceinline__ int div_by(int n, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)n, magic) : n; }
+
+// a * w
+__device__ __forceinline__ float2 gmul(float2 a, float2 w)
+{
+    return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.y, w.x, __fmul_rn(a.x, w.y)));
 }
 
 // W_N^t (forward) or its conjugate (inverse) from the forward table
-__device__ __forceinline__ float2 gtw(const float2 *W, int t, bool inv)
+template <bool INV>
+__device__ __forceinline__ float2 gtw(const float2 *W, int t)
 {
     const float2 w = W[t];
-    return inv ? make_float2(w.x, -w.y) : w;
+    return INV ? make_float2(w.x, -w.y) : w;
 }
 
 // R-point DFT of x in place: y[k] = sum_q x[q] W_R^(q k), W_R^e = W_N^(e N/R)
-template <int R>
-__device__ __forceinline__ void gdft(float2 (&x)[R], const float2 *W, int N, bool inv)
+template <int R, bool INV>
+__device__ __forceinline__ void gdft(float2 (&x)[R], const float2 *W, int N)
 {
     if constexpr (R == 2) {
         const float2 a = x[0], b = x[1];
@@ -69,22 +90,24 @@ __device__ __forceinline__ void gdft(float2 (&x)[R], const float2 *W, int N, boo
         const float2 t0 = make_float2(a.x + c.x, a.y + c.y), t1 = make_float2(a.x - c.x, a.y - c.y);
         const float2 t2 = make_float2(b.x + d.x, b.y + d.y), u = make_float2(b.x - d.x, b.y - d.y);
         // (b - d) times -i (forward) or +i (inverse)
-        const float2 t3 = inv ? make_float2(-u.y, u.x) : make_float2(u.y, -u.x);
+        const float2 t3 = INV ? make_float2(-u.y, u.x) : make_float2(u.y, -u.x);
         x[0] = make_float2(t0.x + t2.x, t0.y + t2.y);
         x[1] = make_float2(t1.x + t3.x, t1.y + t3.y);
         x[2] = make_float2(t0.x - t2.x, t0.y - t2.y);
         x[3] = make_float2(t1.x - t3.x, t1.y - t3.y);
     } else {
         const int st = N / R;
-        float2 y[R];
+        float2 w[R], y[R];
+#pragma unroll
+        for (int q = 1; q < R; ++q) w[q] = gtw<INV>(W, q * st);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             float2 acc = x[0];
 #pragma unroll
             for (int q = 1; q < R; ++q) {
-                const float2 p = gmul(x[q], gtw(W, ((q * k) % R) * st, inv));
-                acc.x += p.x;
-                acc.y += p.y;
+                const float2 p = (q * k) % R ? gmul(x[q], w[(q * k) % R]) : x[q];
+                acc.x = __fadd_rn(acc.x, p.x);
+                acc.y = __fadd_rn(acc.y, p.y);
             }
             y[k] = acc;
         }
@@ -93,40 +116,51 @@ __device__ __forceinline__ void gdft(float2 (&x)[R], const float2 *W, int N, boo
     }
 }
 
-// One stage along one dimension of the plane, for all lines.  Elements of a line are
-// estride apart, lines lstride apart.  DIT (forward): blocks of L points combine R
-// sub-transforms of M = L/R points: inputs at q*M + k1 are twiddled by W_L^(q k1) and
-// transformed, outputs to k1 + M*k2.  DIF (inverse): inputs at m + M*q are transformed
-// and the outputs twiddled by W_L^(m k2), to m + M*k2.  line_fast: consecutive threads
-// take consecutive lines (columns: contiguous addresses) rather than consecutive points.
-template <int R>
-__device__ __forceinline__ void gstage(float2 *buf, int N, int L, int estride, int lines, int lstride,
-                                       const float2 *W, bool inv, bool line_fast)
+// Where a stage works: one dimension of the plane, for all lines.  Elements of a line are
+// estride apart, lines lstride apart.
+struct GLines {
+    int N, estride, lines, lstride;
+    uint32_t by_lines;  // div_by constant of `lines` (used when lines are the fast index)
+    const float2 *W;
+};
+
+// One stage along one dimension.  DIT (forward): blocks of L points combine R sub-transforms of
+// M = L/R points: inputs at q*M + k1 are twiddled by W_L^(q k1) and transformed, outputs to
+// k1 + M*k2.  DIF (inverse): inputs at m + M*q are transformed and the outputs twiddled by
+// W_L^(m k2), to m + M*k2.  LINE_FAST: consecutive threads take consecutive lines (columns:
+// contiguous addresses) rather than consecutive points.  by_m, by_pl: div_by constants of M and
+// of the butterflies per line.
+template <int R, bool INV, bool LINE_FAST>
+__device__ __forceinline__ void gstage(float2 *buf, const GLines &d, int L, uint32_t by_m, uint32_t by_pl)
 {
-    const int M = L / R, tws = N / L, per_line = N / R, total = lines * per_line;
-    for (int b = threadIdx.x; b < total; b += blockDim.x) {
+    const int M = L / R, tws = d.N / L, per_line = d.N / R, total = d.lines * per_line, step = M * d.estride;
+    for (int b = threadIdx.x; b < total; b += kGenThreads) {
         int line, t;
-        if (line_fast) {
-            t = b / lines;
-            line = b - t * lines;
+        if constexpr (LINE_FAST) {
+            t = div_by(b, d.by_lines);
+            line = b - t * d.lines;
         } else {
-            line = b / per_line;
+            line = div_by(b, by_pl);
             t = b - line * per_line;
         }
-        const int blk = t / M, k1 = t - blk * M;
-        float2 *base = buf + (size_t)line * lstride + (size_t)(blk * L + k1) * estride;
-        const size_t step = (size_t)M * estride;
+        const int blk = div_by(t, by_m), k1 = t - blk * M;
+        float2 *base = buf + line * d.lstride + (blk * L + k1) * d.estride;
         float2 x[R];
 #pragma unroll
         for (int q = 0; q < R; ++q) x[q] = base[q * step];
-        if (!inv) {
+        const float2 *w = d.W + k1 * tws;  // q k1 tws < N
+        if constexpr (!INV) {
+            if (M > 1) {
 #pragma unroll
-            for (int q = 1; q < R; ++q) x[q] = gmul(x[q], gtw(W, (q * k1 * tws) % N, false));
-            gdft<R>(x, W, N, false);
+                for (int q = 1; q < R; ++q) x[q] = gmul(x[q], gtw<false>(w, (q - 1) * k1 * tws));
+            }
+            gdft<R, false>(x, d.W, d.N);
         } else {
-            gdft<R>(x, W, N, true);
+            gdft<R, true>(x, d.W, d.N);
+            if (M > 1) {
 #pragma unroll
-            for (int q = 1; q < R; ++q) x[q] = gmul(x[q], gtw(W, (q * k1 * tws) % N, true));
+                for (int q = 1; q < R; ++q) x[q] = gmul(x[q], gtw<true>(w, (q - 1) * k1 * tws));
+            }
         }
 #pragma unroll
         for (int q = 0; q < R; ++q) base[q * step] = x[q];
@@ -134,35 +168,37 @@ __device__ __forceinline__ void gstage(float2 *buf, int N, int L, int estride, i
 }
 
 // A stage of a prime radix above 7 (up to 251): the R-point DFT runs from a local array.
-__device__ __noinline__ void gstage_any(float2 *buf, int R, int N, int L, int estride, int lines, int lstride,
-                                        const float2 *W, bool inv, bool line_fast)
+template <bool INV, bool LINE_FAST>
+__device__ __noinline__ void gstage_any(float2 *buf, int R, const GLines d, int L, uint32_t by_m, uint32_t by_pl)
 {
-    const int M = L / R, tws = N / L, per_line = N / R, total = lines * per_line, st = N / R;
+    const int M = L / R, tws = d.N / L, per_line = d.N / R, total = d.lines * per_line, st = d.N / R;
     float2 x[256];
-    for (int b = threadIdx.x; b < total; b += blockDim.x) {
+    for (int b = threadIdx.x; b < total; b += kGenThreads) {
         int line, t;
-        if (line_fast) {
-            t = b / lines;
-            line = b - t * lines;
+        if constexpr (LINE_FAST) {
+            t = div_by(b, d.by_lines);
+            line = b - t * d.lines;
         } else {
-            line = b / per_line;
+            line = div_by(b, by_pl);
             t = b - line * per_line;
         }
-        const int blk = t / M, k1 = t - blk * M;
-        float2 *base = buf + (size_t)line * lstride + (size_t)(blk * L + k1) * estride;
-        const size_t step = (size_t)M * estride;
+        const int blk = div_by(t, by_m), k1 = t - blk * M, step = M * d.estride;
+        float2 *base = buf + line * d.lstride + (blk * L + k1) * d.estride;
         for (int q = 0; q < R; ++q) {
             x[q] = base[q * step];
-            if (!inv && q > 0) x[q] = gmul(x[q], gtw(W, (q * k1 * tws) % N, false));
+            if (!INV && q > 0) x[q] = gmul(x[q], gtw<false>(d.W, q * k1 * tws));
         }
         for (int k = 0; k < R; ++k) {
             float2 acc = x[0];
+            int e = 0;  // (q k) mod R
             for (int q = 1; q < R; ++q) {
-                const float2 p = gmul(x[q], gtw(W, ((q * k) % R) * st, inv));
-                acc.x += p.x;
-                acc.y += p.y;
+                e += k;
+                if (e >= R) e -= R;
+                const float2 p = gmul(x[q], gtw<INV>(d.W, e * st));
+                acc.x = __fadd_rn(acc.x, p.x);
+                acc.y = __fadd_rn(acc.y, p.y);
             }
-            if (inv && k > 0) acc = gmul(acc, gtw(W, (k * k1 * tws) % N, true));
+            if (INV && k > 0) acc = gmul(acc, gtw<true>(d.W, k * k1 * tws));
             base[k * step] = acc;  // inputs are all in x already
         }
     }
@@ -170,39 +206,42 @@ __device__ __noinline__ void gstage_any(float2 *buf, int R, int N, int L, int es
 
 // ANY: the instance that also carries the local-array stage for primes above 7 (its
 // 2 KB per-thread stack is reserved only when such a window shape is launched)
-template <bool ANY>
-__device__ __forceinline__ void gstage_r(float2 *buf, int R, int N, int L, int estride, int lines, int lstride,
-                                         const float2 *W, bool inv, bool line_fast)
+template <bool ANY, bool INV, bool LF>
+__device__ __forceinline__ void gstage_r(float2 *buf, int R, const GLines &d, int L, uint32_t by_m, uint32_t by_pl)
 {
     switch (R) {
-    case 2: gstage<2>(buf, N, L, estride, lines, lstride, W, inv, line_fast); break;
-    case 3: gstage<3>(buf, N, L, estride, lines, lstride, W, inv, line_fast); break;
-    case 4: gstage<4>(buf, N, L, estride, lines, lstride, W, inv, line_fast); break;
-    case 5: gstage<5>(buf, N, L, estride, lines, lstride, W, inv, line_fast); break;
-    case 7: gstage<7>(buf, N, L, estride, lines, lstride, W, inv, line_fast); break;
+    case 2: gstage<2, INV, LF>(buf, d, L, by_m, by_pl); break;
+    case 3: gstage<3, INV, LF>(buf, d, L, by_m, by_pl); break;
+    case 4: gstage<4, INV, LF>(buf, d, L, by_m, by_pl); break;
+    case 5: gstage<5, INV, LF>(buf, d, L, by_m, by_pl); break;
+    case 7: gstage<7, INV, LF>(buf, d, L, by_m, by_pl); break;
     default:
-        if constexpr (ANY) gstage_any(buf, R, N, L, estride, lines, lstride, W, inv, line_fast);
+        if constexpr (ANY) {
+            if (R == 11) gstage<11, INV, LF>(buf, d, L, by_m, by_pl);
+            else if (R == 13) gstage<13, INV, LF>(buf, d, L, by_m, by_pl);
+            else gstage_any<INV, LF>(buf, R, d, L, by_m, by_pl);
+        }
         break;
     }
 }
 
 // Forward (DIT, innermost radix first) or inverse (DIF, outermost first) transform of
 // every line of one dimension.  f: radices, outermost first.
-template <bool ANY>
-__device__ void gfft_dim(float2 *buf, const int *f, int nf, int N, int estride, int lines, int lstride,
-                         const float2 *W, bool inv, bool line_fast)
+template <bool ANY, bool INV, bool LF>
+__device__ void gfft_dim(float2 *buf, const int *f, int nf, const uint32_t *by_m, const uint32_t *by_pl,
+                         const GLines &d)
 {
-    if (!inv) {
+    if constexpr (!INV) {
         int L = 1;
         for (int s = nf - 1; s >= 0; --s) {
             L *= f[s];
-            gstage_r<ANY>(buf, f[s], N, L, estride, lines, lstride, W, false, line_fast);
+            gstage_r<ANY, false, LF>(buf, f[s], d, L, by_m[s], by_pl[s]);
             __syncthreads();
         }
     } else {
-        int L = N;
+        int L = d.N;
         for (int s = 0; s < nf; ++s) {
-            gstage_r<ANY>(buf, f[s], N, L, estride, lines, lstride, W, true, line_fast);
+            gstage_r<ANY, true, LF>(buf, f[s], d, L, by_m[s], by_pl[s]);
             __syncthreads();
             L /= f[s];
         }
@@ -260,170 +299,254 @@ __device__ __forceinline__ void gblock_best(float &v, int &i, int &cnt, float *r
     }
 }
 
+// The search region's local maxima, top-K list per thread (rows by warp, columns by lane, so a
+// thread meets them in ascending index order), then per warp, then over the warps: pv, pi get
+// the Nps best.  Returns the count (thread 0).
+template <int K, class Plane>
+__device__ __forceinline__ int gpeaks(const Plane &P, int Nps, int nx, int ilo, int ihi, int jlo, int jhi, float *pv,
+                                      int *pi, PeakPart *parts)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float tiny = __int_as_float(1);  // v >= max(neighbours, tiny)  <=>  v > 0 and a local maximum
+    float tv[K];
+    int ti[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        tv[k] = -1.f;
+        ti[k] = INT_MAX;
+    }
+    int cnt = 0;
+    for (int j = jlo + warp; j <= jhi; j += kGenWarps)
+        for (int i = ilo + lane; i <= ihi; i += 32) {
+            const float v = P(i, j);
+            const float m = fmaxf(fmaxf(P(i - 1, j), P(i + 1, j)), fmaxf(fmaxf(P(i, j - 1), P(i, j + 1)), tiny));
+            if (v >= m) {
+                ++cnt;
+                topk_insert<K>(tv, ti, v, j * nx + i);
+            }
+        }
+    cnt = warp_sum(cnt);
+    float v;
+    int idx;
+    peak_select<K>(Nps, lane, tv, ti, v, idx);
+    if (lane < Nps) {
+        parts[warp].v[lane] = v;
+        parts[warp].idx[lane] = idx;
+    }
+    if (lane == 0) parts[warp].cnt = cnt;
+    __syncthreads();
+    cnt = 0;
+    if (warp == 0) {
+        // two list entries per lane hold the warps' up to 8 x 8 picks, best first
+        static_assert(kGenWarps * 8 <= 64, "two entries per lane");
+        float mv[2] = {-1.f, -1.f};
+        int mi[2] = {INT_MAX, INT_MAX};
+        for (int e = lane; e < kGenWarps * Nps; e += 32) {
+            const int q = e / Nps, k = e - q * Nps;
+            const float ev = parts[q].v[k];
+            const int ei = parts[q].idx[k];
+            if (gbetter(ev, ei, mv[0], mi[0])) {
+                mv[1] = mv[0];
+                mi[1] = mi[0];
+                mv[0] = ev;
+                mi[0] = ei;
+            } else {
+                mv[1] = ev;
+                mi[1] = ei;
+            }
+        }
+        peak_select<2>(Nps, lane, mv, mi, v, idx);
+        if (lane < Nps) {
+            pv[lane] = v;
+            pi[lane] = idx;
+        }
+        cnt = warp_sum(lane < kGenWarps ? parts[lane].cnt : 0);
+    }
+    return cnt;
+}
+
 }  // namespace
 
-template <bool DEF, bool ANY>
-__global__ void __launch_bounds__(kGenThreads) xcorr_generic_kernel(const XcorrArgs a, const GenericPlan pl,
-                                                                    float2 *gplane)
+// SMEM: the plane in shared memory (known at compile time, so that its accesses are 32-bit
+// shared-memory instructions rather than generic ones).
+template <bool DEF, bool ANY, bool SMEM>
+__global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel(const XcorrArgs a,
+                                                                                 const GenericPlan pl, float2 *gplane)
 {
     const GridGeom &g = a.g;
-    const int nx = g.ws_x, ny = g.ws_y, N = nx * ny, tid = threadIdx.x;
+    const int nx = g.ws_x, ny = g.ws_y, N = nx * ny, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     extern __shared__ __align__(16) unsigned char gsm[];
+    __shared__ PeakPart parts[kGenWarps];
     float2 *Wx = reinterpret_cast<float2 *>(gsm);
     float2 *Wy = Wx + nx;
     int *Sx = reinterpret_cast<int *>(Wy + ny);  // shifted column -> storage column
     int *Sy = Sx + nx;                            // shifted row -> storage row offset
-    float *rv = reinterpret_cast<float *>(Sy + ny);
+    int *Px = Sy + ny;                            // column -> digit-reversed column
+    int *Py = Px + nx;                            // row -> digit-reversed row offset
+    float *rv = reinterpret_cast<float *>(Py + ny);
     int *ri = reinterpret_cast<int *>(rv + 32);
     int *rc = ri + 32;
     float *pv = reinterpret_cast<float *>(rc + 32);  // the window's picks
     int *pi = reinterpret_cast<int *>(pv + g.Nps);
-    float2 *plane = pl.in_smem ? reinterpret_cast<float2 *>(
-                                     gsm + (((size_t)(nx + ny) * 16 + 96 * 4 + (size_t)g.Nps * 8 + 15) & ~(size_t)15))
-                               : gplane + (size_t)blockIdx.x * N;
+    float2 *plane;
+    if constexpr (SMEM)
+        plane = reinterpret_cast<float2 *>(gsm + (((size_t)(nx + ny) * 16 + 96 * 4 + (size_t)g.Nps * 8 + 15) & ~(size_t)15));
+    else
+        plane = gplane + (size_t)blockIdx.x * N;
 
-    // tables: forward twiddles (FP64, rounded once) and the shifted-index maps
-    for (int t = tid; t < nx; t += blockDim.x) {
+    // tables: forward twiddles (FP64, rounded once) and the index maps
+    for (int t = tid; t < nx; t += kGenThreads) {
         double s, c;
         sincospi(2.0 * (double)t / (double)nx, &s, &c);
         Wx[t] = make_float2((float)c, (float)(-s));
         Sx[t] = gperm((t + nx / 2) % nx, pl.fx, pl.nfx, nx);
+        Px[t] = gperm(t, pl.fx, pl.nfx, nx);
     }
-    for (int t = tid; t < ny; t += blockDim.x) {
+    for (int t = tid; t < ny; t += kGenThreads) {
         double s, c;
         sincospi(2.0 * (double)t / (double)ny, &s, &c);
         Wy[t] = make_float2((float)c, (float)(-s));
         Sy[t] = gperm((t + ny / 2) % ny, pl.fy, pl.nfy, ny) * nx;
+        Py[t] = gperm(t, pl.fy, pl.nfy, ny) * nx;
     }
     __syncthreads();
 
-    const float tiny = __int_as_float(1);  // v >= max(neighbours, tiny)  <=>  v > 0 and a local maximum
+    const float tiny = __int_as_float(1);
     const int ilo = g.bx > 1 ? g.bx : 1, ihi = min(nx - 1 - g.bx, nx - 2);
     const int jlo = g.by > 1 ? g.by : 1, jhi = min(ny - 1 - g.by, ny - 2);
     const int rw = ihi - ilo + 1, rh = jhi - jlo + 1, region = (rw > 0 && rh > 0) ? rw * rh : 0;
+    const GLines rows = {nx, 1, ny, nx, 0u, Wx}, cols = {ny, nx, nx, 1, pl.dx, Wy};
 
     for (int w = a.w_first + blockIdx.x; w < a.w_end; w += gridDim.x) {
         const int iy = w / g.Nx_vec, ix = w - iy * g.Nx_vec;
-        // ---- load at the digit-reversed positions of the forward transform ----
-        for (int t = tid; t < N; t += blockDim.x) {
-            const int r = t / nx, i = t - r * nx;
-            const int x0 = ix * g.sp_x - g.Nx_left + a.f1.mx, y1 = iy * g.sp_y + r - g.Ny_left + a.f1.my;
-            const float v1 = (float)a.f1.base[(size_t)y1 * a.f1.pitch + x0 + i];
-            float v2;
-            if constexpr (DEF) v2 = a.def[(size_t)(iy * g.sp_y + r) * a.def_pitch + ix * g.sp_x + i];
-            else v2 = (float)a.f2.base[(size_t)y1 * a.f2.pitch + x0 + i];
-            plane[(size_t)gperm(r, pl.fy, pl.nfy, ny) * nx + gperm(i, pl.fx, pl.nfx, nx)] = make_float2(v1, v2);
+        // ---- load at the digit-reversed positions of the forward transform: rows by warp ----
+        {
+            const size_t px = (size_t)(iy * g.sp_y - g.Ny_left + a.f1.my) * a.f1.pitch + ix * g.sp_x - g.Nx_left + a.f1.mx;
+            const uint8_t *p1 = a.f1.base + px, *p2 = a.f2.base + px;
+            const float *pd = DEF ? a.def + (size_t)(iy * g.sp_y) * a.def_pitch + ix * g.sp_x : nullptr;
+            for (int r = warp; r < ny; r += kGenWarps) {
+                float2 *row = plane + Py[r];
+#pragma unroll 4
+                for (int i = lane; i < nx; i += 32) {
+                    const float v1 = (float)p1[(size_t)r * a.f1.pitch + i];
+                    float v2;
+                    if constexpr (DEF) v2 = pd[(size_t)r * a.def_pitch + i];
+                    else v2 = (float)p2[(size_t)r * a.f2.pitch + i];
+                    row[Px[i]] = make_float2(v1, v2);
+                }
+            }
         }
         __syncthreads();
         // ---- forward 2D transform: rows (x), then columns (y) ----
-        gfft_dim<ANY>(plane, pl.fx, pl.nfx, nx, 1, ny, nx, Wx, false, false);
-        gfft_dim<ANY>(plane, pl.fy, pl.nfy, ny, nx, nx, 1, Wy, false, true);
+        gfft_dim<ANY, false, false>(plane, pl.fx, pl.nfx, pl.mx, pl.px, rows);
+        gfft_dim<ANY, false, true>(plane, pl.fy, pl.nfy, pl.my, pl.py, cols);
         // ---- cross spectrum, in place over (k, -k) pairs.  Z(0,0) = (sum f1, sum f2) is
         //      exactly zero iff a frame's window is all zero; the reference's correlation is
         //      then exactly 0 (no candidate), so the spectrum is set to 0 ----
         const float2 dc = plane[0];
         const bool dead = dc.x == 0.f || dc.y == 0.f;
         __syncthreads();  // every thread has read the DC term before it is overwritten
-        for (int t = tid; t < N; t += blockDim.x) {
-            const int ky = t / nx, kx = t - ky * nx;
-            const int tm = ((ny - ky) % ny) * nx + (nx - kx) % nx;
-            if (tm < t) continue;
-            const float2 A = plane[t], M = plane[tm];
-            const float2 C = dead ? make_float2(0.f, 0.f)
-                                  : make_float2(0.5f * (A.x * M.y + A.y * M.x),
-                                                0.25f * ((M.x * M.x + M.y * M.y) - (A.x * A.x + A.y * A.y)));
-            plane[t] = C;
-            if (tm != t) plane[tm] = make_float2(C.x, -C.y);
+        for (int ky = warp; ky <= ny / 2; ky += kGenWarps) {
+            const int my = ky ? ny - ky : 0;
+            for (int kx = lane; kx < nx; kx += 32) {
+                const int mx = kx ? nx - kx : 0, t = ky * nx + kx, tm = my * nx + mx;
+                if (tm < t) continue;
+                const float2 A = plane[t], M = plane[tm];
+                const float im2 = __fmaf_rn(A.y, M.x, __fmul_rn(A.x, M.y));
+                const float pw = __fsub_rn(__fmaf_rn(M.y, M.y, __fmul_rn(M.x, M.x)), __fmaf_rn(A.y, A.y, __fmul_rn(A.x, A.x)));
+                const float2 C = dead ? make_float2(0.f, 0.f) : make_float2(0.5f * im2, 0.25f * pw);
+                plane[t] = C;
+                if (tm != t) plane[tm] = make_float2(C.x, -C.y);
+            }
         }
         __syncthreads();
         // ---- inverse 2D transform (natural in, digit-reversed out), then |.|/N ----
-        gfft_dim<ANY>(plane, pl.fy, pl.nfy, ny, nx, nx, 1, Wy, true, true);
-        gfft_dim<ANY>(plane, pl.fx, pl.nfx, nx, 1, ny, nx, Wx, true, false);
-        for (int t = tid; t < N; t += blockDim.x) {
+        gfft_dim<ANY, true, true>(plane, pl.fy, pl.nfy, pl.my, pl.py, cols);
+        gfft_dim<ANY, true, false>(plane, pl.fx, pl.nfx, pl.mx, pl.px, rows);
+        for (int t = tid; t < N; t += kGenThreads) {
             const float2 z = plane[t];
-            plane[t].x = __fdiv_rn(sqrtf(z.x * z.x + z.y * z.y), (float)N);
+            plane[t].x = __fdiv_rn(sqrtf(__fmaf_rn(z.x, z.x, __fmul_rn(z.y, z.y))), (float)N);
         }
         __syncthreads();
         auto P = [&](int i, int j) -> float { return plane[Sy[j] + Sx[i]].x; };
         if (a.cc_dump) {
             float *dst = a.cc_dump + (size_t)(w - a.w_first) * N;
-            for (int t = tid; t < N; t += blockDim.x) {
-                const int j = t / nx, i = t - j * nx;
-                dst[t] = P(i, j);
-            }
+            for (int j = warp; j < ny; j += kGenWarps)
+                for (int i = lane; i < nx; i += 32) dst[j * nx + i] = P(i, j);
             __syncthreads();
             continue;
         }
-        // ---- peaks: Npeak_save rounds of a block arg-max over the local maxima ----
-        float prev_v = FLT_MAX;
-        int prev_i = -1, cnt = 0;
-        for (int k = 0; k < g.Nps; ++k) {
-            float bv = -1.f;
-            int bi = INT_MAX, c = 0;
-            if (prev_v > 0.f) {
-                for (int t = tid; t < region; t += blockDim.x) {
-                    const int jj = t / rw, j = jlo + jj, i = ilo + (t - jj * rw);
-                    const float v = P(i, j);
-                    const float m = fmaxf(fmaxf(P(i - 1, j), P(i + 1, j)), fmaxf(fmaxf(P(i, j - 1), P(i, j + 1)), tiny));
-                    if (!(v >= m)) continue;
-                    if (k == 0) ++c;
-                    const int idx = j * nx + i;
-                    if (gbetter(prev_v, prev_i, v, idx) && gbetter(v, idx, bv, bi)) {
-                        bv = v;
-                        bi = idx;
+        int cnt = 0;
+        if (g.Nps <= 4) {
+            cnt = gpeaks<4>(P, g.Nps, nx, ilo, ihi, jlo, jhi, pv, pi, parts);
+        } else if (g.Nps <= 8) {
+            cnt = gpeaks<8>(P, g.Nps, nx, ilo, ihi, jlo, jhi, pv, pi, parts);
+        } else {
+            // Npeak_save rounds of a block arg-max over the local maxima
+            float prev_v = FLT_MAX;
+            int prev_i = -1;
+            for (int k = 0; k < g.Nps; ++k) {
+                float bv = -1.f;
+                int bi = INT_MAX, c = 0;
+                if (prev_v > 0.f) {
+                    for (int t = tid; t < region; t += kGenThreads) {
+                        const int jj = t / rw, j = jlo + jj, i = ilo + (t - jj * rw);
+                        const float v = P(i, j);
+                        const float m = fmaxf(fmaxf(P(i - 1, j), P(i + 1, j)), fmaxf(fmaxf(P(i, j - 1), P(i, j + 1)), tiny));
+                        if (!(v >= m)) continue;
+                        if (k == 0) ++c;
+                        const int idx = j * nx + i;
+                        if (gbetter(prev_v, prev_i, v, idx) && gbetter(v, idx, bv, bi)) {
+                            bv = v;
+                            bi = idx;
+                        }
                     }
                 }
+                gblock_best(bv, bi, c, rv, ri, rc);
+                if (k == 0) cnt = c;
+                if (tid == 0) {
+                    pv[k] = bv;
+                    pi[k] = bi;
+                }
+                prev_v = bv;
+                prev_i = bi;
             }
-            gblock_best(bv, bi, c, rv, ri, rc);
-            if (k == 0) cnt = c;
-            if (tid == 0) {
-                pv[k] = bv;
-                pi[k] = bi;
-            }
-            prev_v = bv;
-            prev_i = bi;
         }
         __syncthreads();
-        // ---- fit and store (same arithmetic as the fused kernels' peak_fit_store) ----
-        const float pred_x = a.pred_x[w], pred_y = a.pred_y[w];
-        for (int k = tid; k < g.Nps; k += blockDim.x) {
-            const float v = pv[k];
-            const int idx = pi[k];
-            float ox = 0.f, oy = 0.f;
+        // ---- fit and store; the x and y halves of a pick on neighbouring lanes ----
+        for (int e0 = tid & ~31; e0 < 2 * g.Nps; e0 += kGenThreads) {
+            const int e = e0 + lane, k = e >> 1, comp = e & 1;
+            const bool live = k < g.Nps;
+            const float v = live ? pv[k] : -1.f;
+            const int idx = live ? pi[k] : 0;
+            float o = 0.f;
             bool ok = false;
             if (v > 0.f) {
                 const int j = idx / nx, i = idx - j * nx;
                 if (i != 0 && i != nx - 1 && j != 0 && j != ny - 1) {
-                    float sh[2];
-                    for (int comp = 0; comp < 2; ++comp) {
-                        const float f0 = comp ? P(i, j - 1) : P(i - 1, j);
-                        const float f2 = comp ? P(i, j + 1) : P(i + 1, j);
-                        const double dv = (double)v * (double)v;
-                        const float nn = logf(f0) - logf(f2);
-                        const double den = log(((double)f0 * (double)f2) / dv);
-                        sh[comp] = (float)((double)nn / den / 2.0);
-                    }
-                    ox = (float)i + sh[0] - (float)nx / 2 + pred_x;
-                    oy = (float)j + sh[1] - (float)ny / 2 + pred_y;
+                    const float f0 = comp ? P(i, j - 1) : P(i - 1, j);
+                    const float f2 = comp ? P(i, j + 1) : P(i + 1, j);
+                    const double dv = (double)v * (double)v;
+                    const float nn = logf(f0) - logf(f2);
+                    const double den = log(((double)f0 * (double)f2) / dv);
+                    const float sh = (float)((double)nn / den / 2.0);
+                    o = comp ? (float)j + sh - (float)ny / 2 + a.pred_y[w] : (float)i + sh - (float)nx / 2 + a.pred_x[w];
                     ok = true;
-                    if (ox < g.lx1 || ox > g.lx2 || oy < g.ly1 || oy > g.ly2) {
-                        ok = false;
-                        ox = 0.f;
-                        oy = 0.f;
-                    }
-                    if (isnan(ox) || isnan(oy) || isinf(ox) || isinf(oy)) {
-                        ok = false;
-                        ox = 0.f;
-                        oy = 0.f;
-                    }
                 }
             }
-            const size_t o = (size_t)w * g.Nps + k;
-            a.cdx[o] = ox;
-            a.cdy[o] = oy;
-            a.cvalid[o] = ok ? 1 : 0;
-            a.pidx[o] = (v > 0.f) ? idx : -1;
-            a.pval[o] = (v > 0.f) ? v : 0.f;
+            float other = __shfl_xor_sync(0xffffffffu, o, 1);
+            if (ok) ok = comp ? peak_limits(g, other, o) : peak_limits(g, o, other);
+            if (live) {
+                const size_t q = (size_t)w * g.Nps + k;
+                if (comp == 0) {
+                    a.cdx[q] = o;
+                    a.cvalid[q] = ok ? 1 : 0;
+                    a.pidx[q] = (v > 0.f) ? idx : -1;
+                } else {
+                    a.cdy[q] = o;
+                    a.pval[q] = (v > 0.f) ? v : 0.f;
+                }
+            }
         }
         if (tid == 0) a.count[w] = cnt;
         __syncthreads();
@@ -463,8 +586,18 @@ GenericPlan generic_plan(int wsx, int wsy)
     pl.nfy = radices(wsy, pl.fy);
     pl.in_smem = wsx * wsy <= kGenSmemPlane ? 1 : 0;
     pl.any = 0;
-    for (int s = 0; s < pl.nfx; ++s) pl.any |= pl.fx[s] > 7;
-    for (int s = 0; s < pl.nfy; ++s) pl.any |= pl.fy[s] > 7;
+    auto constants = [&](int n, const int *f, int nf, uint32_t *by_m, uint32_t *by_pl) {
+        int M = n;
+        for (int s = 0; s < nf; ++s) {
+            pl.any |= f[s] > 7;
+            M /= f[s];
+            by_m[s] = div_magic32(M);
+            by_pl[s] = div_magic32(n / f[s]);
+        }
+    };
+    constants(wsx, pl.fx, pl.nfx, pl.mx, pl.px);
+    constants(wsy, pl.fy, pl.nfy, pl.my, pl.py);
+    pl.dx = div_magic32(wsx);
     return pl;
 }
 
@@ -499,17 +632,24 @@ cudaError_t launch_xcorr_generic(const XcorrArgs &a, bool deformed, float2 *work
     if (ctas > n) ctas = n;
     cudaError_t e = cudaSuccess;
     auto go = [&](auto kern) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the largest any launch asks for: a captured launch of another grid's (larger) windows
+        // keeps running under the attribute set last
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
         if (e != cudaSuccess) return;
         kern<<<ctas, kGenThreads, smem, s>>>(a, pl, workspace);
         e = cudaGetLastError();
     };
+    auto pick = [&](auto any, auto in_smem) {
+        constexpr bool A = decltype(any)::value, S = decltype(in_smem)::value;
+        if (deformed) go(xcorr_generic_kernel<true, A, S>);
+        else go(xcorr_generic_kernel<false, A, S>);
+    };
     if (pl.any) {
-        if (deformed) go(xcorr_generic_kernel<true, true>);
-        else go(xcorr_generic_kernel<false, true>);
+        if (pl.in_smem) pick(std::true_type{}, std::true_type{});
+        else pick(std::true_type{}, std::false_type{});
     } else {
-        if (deformed) go(xcorr_generic_kernel<true, false>);
-        else go(xcorr_generic_kernel<false, false>);
+        if (pl.in_smem) pick(std::false_type{}, std::true_type{});
+        else pick(std::false_type{}, std::false_type{});
     }
     return e;
 }
