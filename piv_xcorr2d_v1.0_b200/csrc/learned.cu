@@ -724,64 +724,326 @@ __global__ void __launch_bounds__(128) conv_bwd_data_kernel(const ConvBwdData c)
     }
 }
 
-// dW[co][ci][tap] and db[co]: one CTA per (input channel, COC output channels), threads
-// over the N*Ho*Wo output pixels, then a block reduction.  Overwrites its outputs.
+// The same for cout a multiple of 8 as a register-tiled product.  A warp takes 8 runs of 8 pixels
+// (of one row each) x 32 input channels: a thread holds 8 pixels x 8 channels, so a tap of an
+// output channel costs 2 16-byte weight loads and a third of 3 gradient loads for 64 FMAs (one
+// pixel x 32 channels per thread took 8 weight loads for 32 FMAs and was bound by them).  The
+// 4 warps of a CTA share the staged weights of 8 output channels; each warp stages its own runs'
+// 3 x 10 gradient values of those channels.  Stride 2 reads the gradient as if zeros lay between
+// its pixels, and skips the products whose column is such a zero.  The output channels are split
+// over blockIdx.z where the pixels alone leave the GPU idle (the coarse levels): each split
+// overwrites its own sums in din, which split_grad_kernel adds up in split order.  The 12 layers
+// at 64 x 31 x 31: 1.25 -> 0.63 ms (0.19 ms of FMAs), split_grad 0.12 -> 0.15 ms.
+constexpr int kBdRuns = 8, kBdCo = 8, kBdRow = 12, kBdRun = 3 * kBdRow, kBdWarps = 4;
+
+struct BwdDataSmem {
+    float w[kBdCo][9][32];
+    float g[kBdWarps][kBdCo][kBdRuns][kBdRun];
+};
+
+template <int STRIDE>
+__global__ void __launch_bounds__(32 * kBdWarps, 4) conv_bwd_data_tile_kernel(const ConvBwdData c, int co_per_split)
+{
+    extern __shared__ __align__(16) uint8_t bd_raw[];
+    BwdDataSmem &S = *reinterpret_cast<BwdDataSmem *>(bd_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ci0 = blockIdx.y * 32;
+    const int RW = (c.Win + 7) >> 3, runs = c.N * c.Hin * RW;
+    // this thread's run and its 8 channels; lanes of a run are neighbours
+    const int q = lane & 3, rl = lane >> 2;
+    const int run = (blockIdx.x * kBdWarps + warp) * kBdRuns + rl;
+    const bool live = run < runs;
+    const int yy = live ? run / RW : 0, rx = live ? run - yy * RW : 0;
+    const int n = yy / c.Hin, y = yy - n * c.Hin, x = rx * 8;
+    // the run's 30 gradient values: 8 per lane, their offsets in an output plane (-1: zero)
+    int off[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int e = q + 4 * k, r = e / 10, i = e - r * 10;
+        int gy = y - 1 + r, gx = x - 1 + i;
+        bool ok = live && e < 30 && gy >= 0 && gx >= 0;
+        if (STRIDE == 2) {
+            ok = ok && !(gy & 1) && !(gx & 1);
+            gy >>= 1;
+            gx >>= 1;
+        }
+        off[k] = ok && gy < c.Ho && gx < c.Wo ? gy * c.Wo + gx : -1;
+    }
+    const int plane = c.Ho * c.Wo;
+    const float *gn = c.g + (size_t)n * c.cout * plane;
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[i][k] = 0.f;
+    const int co_end = min(c.cout, (int)(blockIdx.z + 1) * co_per_split);
+    for (int co0 = blockIdx.z * co_per_split; co0 < co_end; co0 += kBdCo) {
+        __syncthreads();
+        const float *src = gn + (size_t)co0 * plane;
+#pragma unroll
+        for (int co = 0; co < kBdCo; ++co) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = off[k] >= 0 ? __ldg(src + off[k]) : 0.f;
+            src += plane;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int e = q + 4 * k, r = e / 10, i = e - r * 10;
+                if (e < 30) S.g[warp][co][rl][r * kBdRow + i] = v[k];
+            }
+        }
+        // the weights [co][ci][tap] of 8 x 32 channels: 288 of an output channel lie together
+        for (int e = threadIdx.x; e < 288; e += 32 * kBdWarps) {
+            const int ci = e / 9, tap = e - ci * 9;
+            const bool ok = ci0 + ci < c.cin;
+            const __nv_bfloat16 *w = c.w + ((size_t)co0 * c.cin + ci0) * 9 + e;
+#pragma unroll
+            for (int co = 0; co < kBdCo; ++co) S.w[co][tap][ci] = ok ? __bfloat162float(w[(size_t)co * c.cin * 9]) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int co = 0; co < kBdCo; ++co) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                // gradient row y - 1 + r meets kernel row 2 - r
+                const float *gp = &S.g[warp][co][rl][r * kBdRow];
+                const float4 g0 = *reinterpret_cast<const float4 *>(gp), g1 = *reinterpret_cast<const float4 *>(gp + 4);
+                const float2 g2 = *reinterpret_cast<const float2 *>(gp + 8);
+                const float gv[10] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w, g2.x, g2.y};
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx) {
+                    const float4 *wp = reinterpret_cast<const float4 *>(&S.w[co][(2 - r) * 3 + kx][8 * q]);
+                    const float4 wa = wp[0], wb = wp[1];
+                    const float wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if (STRIDE == 2 && (i - kx) % 2 == 0) continue;  // column x - 1 + i + 2 - kx is odd: a zero
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) acc[i][k] = fmaf(wv[k], gv[i + 2 - kx], acc[i][k]);
+                    }
+                }
+            }
+        }
+    }
+    if (!live) return;
+    float *out = c.din + (size_t)blockIdx.z * c.N * c.cin * c.Hin * c.Win;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int ci = ci0 + 8 * q + k;
+        if (ci >= c.cin) break;
+        float *dst = out + (((size_t)n * c.cin + ci) * c.Hin + y) * c.Win + x;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (x + i < c.Win) dst[i] = acc[i][k];
+    }
+}
+
+// dW[co][ci][tap] and db[co] as a register-tiled product over the output pixels.  A CTA takes 8
+// input channels x 32 output channels; its warps share out segments of up to 32 pixels (rows of one
+// image), and blockIdx.z splits them further.  A thread holds 4 output x 2 input channels x 9 taps
+// (72 sums): a pixel costs one 16-byte gradient load and, sliding along the row, three 8-byte input
+// loads for 72 FMAs.  (A CTA per input channel and 8 output channels with every pixel's 9 taps
+// gathered from global memory took four times as long.)  Each warp stages its segment's rows in its
+// own shared memory; the warps' sums meet there at the end, the splits' in bwd_w_finish_kernel, in
+// a fixed order.  The 13 layers at 64 x 31 x 31: 2.94 -> 0.79 ms (0.23 ms of FMAs at the FP32
+// peak; 64 % of the instructions are FMAs, 72 % of the issue slots used), finish 0.05 ms.
+constexpr int kBwPx = 32, kBwX = 1536, kBwG = 32 * (kBwPx + 1);
+
 struct ConvBwdW {
     ConvIn in;
     int N, Ho, Wo, stride, cout;
     const float *g;
-    float *dw, *db;
+    float *part;    // [splits][cout * cin * 9 + cout]: weight sums, then bias sums
+    int splits;
+    int segw, segh, per_row, per_img, segs;  // segment width and rows, segments per row / image / in all
 };
 
-template <int COC>
-__global__ void __launch_bounds__(256) conv_bwd_w_kernel(const ConvBwdW c)
+// Segments of up to kBwPx pixels: parts of a row, or several whole rows of a narrow image.
+inline void bwd_w_segments(ConvBwdW &c)
 {
-    constexpr int NV = COC * 10;  // 9 taps + bias per output channel
-    __shared__ float red[8][NV];
-    const int ci = blockIdx.x, co0 = blockIdx.y * COC;
+    c.segw = std::min(c.Wo, c.stride == 2 ? kBwPx / 2 : kBwPx);
+    c.per_row = (c.Wo + c.segw - 1) / c.segw;
+    c.segh = 1;
+    if (c.per_row == 1)
+        while ((c.segh + 1) * c.Wo <= kBwPx && c.segh < c.Ho &&
+               (((c.segh * c.stride + 3) * ((c.Wo - 1) * c.stride + 3)) | 1) * 8 <= kBwX)
+            ++c.segh;
+    c.per_img = ((c.Ho + c.segh - 1) / c.segh) * c.per_row;
+    c.segs = c.N * c.per_img;
+}
+
+constexpr size_t kBwSmem = (size_t)8 * (kBwX + kBwG) * sizeof(float);
+
+template <int STRIDE>
+__global__ void __launch_bounds__(256, 2) conv_bwd_w_kernel(const ConvBwdW c)
+{
+    extern __shared__ __align__(16) float bw_sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ci0 = blockIdx.x * 8, co0 = blockIdx.y * 32;
     const int cin = c.in.ca + c.in.cb;
-    const int HW = c.Ho * c.Wo, npix = c.N * HW;
-    float acc[COC][10];
+    float *xs = bw_sm + warp * (kBwX + kBwG), *gs = xs + kBwX;
+    const int XW = (c.segw - 1) * STRIDE + 3;               // staged input columns
+    const int XP = ((c.segh - 1) * STRIDE + 3) * XW | 1;    // cells of a channel pair (odd: no bank conflicts)
+    const int GP = c.segh * c.segw | 1;                     // cells of four output channels
+    const int p = lane & 3, cg = lane >> 2;                 // this thread's channel pair and output group
+    float acc[4][2][9];
 #pragma unroll
-    for (int k = 0; k < COC; ++k)
+    for (int o = 0; o < 4; ++o)
 #pragma unroll
-        for (int t = 0; t < 10; ++t) acc[k][t] = 0.f;
-    for (int q = threadIdx.x; q < npix; q += 256) {
-        const int n = q / HW, p = q - n * HW;
-        const int oy = p / c.Wo, ox = p - oy * c.Wo;
-        int oa[9], ob[9];
-        conv_taps(c.in, oy, ox, c.stride, true, oa, ob);
-        float x[9];
-        conv_gather(c.in, n, ci, oa, ob, x);
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int k = 0; k < COC; ++k) {
-            const int co = co0 + k;
-            const float gv = co < c.cout ? __ldg(c.g + ((size_t)n * c.cout + co) * HW + p) : 0.f;
+            for (int t = 0; t < 9; ++t) acc[o][i][t] = 0.f;
+    float bias = 0.f;  // output channel co0 + lane
+    // the 8 channels lie in one of the two inputs (a's channel counts with a b beside it are
+    // multiples of 8); e / XW and e / segw by multiply-high (e < 2^16)
+    const bool in_b = ci0 >= c.in.ca, up = !in_b && c.in.up;
+    const int src_w = in_b ? c.in.Win : c.in.Wa, src_plane = in_b ? c.in.Hin * c.in.Win : c.in.Ha * c.in.Wa;
+    const float *src = in_b ? c.in.b + (size_t)(ci0 - c.in.ca) * src_plane : c.in.a + (size_t)ci0 * src_plane;
+    const size_t src_n = (size_t)(in_b ? c.in.cb : c.in.ca) * src_plane;
+    const int channels = min(8, cin - ci0), outs = min(32, c.cout - co0), g_plane = c.Ho * c.Wo;
+    const uint32_t by_xw = 0xffffffffu / XW + 1, by_segw = c.segw > 1 ? 0xffffffffu / c.segw + 1 : 0;
+    for (int seg = blockIdx.z * 8 + warp; seg < c.segs; seg += c.splits * 8) {
+        const int n = seg / c.per_img, rem = seg - n * c.per_img;
+        const int sy = rem / c.per_row, y0 = sy * c.segh, x0 = (rem - sy * c.per_row) * c.segw;
+        const int h = min(c.segh, c.Ho - y0), w = min(c.segw, c.Wo - x0);
+        __syncwarp();
+        // input rows y0 * STRIDE - 1 .., columns x0 * STRIDE - 1 .., 8 channels as 4 pairs per cell
+        const int xcells = ((h - 1) * STRIDE + 3) * XW;
+        const float *xin = src + (size_t)n * src_n;
+        for (int e = lane; e < xcells; e += 32) {
+            const int r = (int)__umulhi((uint32_t)e, by_xw), i = e - r * XW;
+            const int iy = y0 * STRIDE - 1 + r, ix = x0 * STRIDE - 1 + i;
+            const bool ok = iy >= 0 && iy < c.in.Hin && ix >= 0 && ix < c.in.Win;
+            const int o = up ? (iy >> 1) * src_w + (ix >> 1) : iy * src_w + ix;
+            float v[8];
 #pragma unroll
-            for (int t = 0; t < 9; ++t) acc[k][t] = fmaf(gv, x[t], acc[k][t]);
-            acc[k][9] += gv;
+            for (int k = 0; k < 8; ++k) v[k] = ok && k < channels ? __ldg(xin + (k * src_plane + o)) : 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) reinterpret_cast<float2 *>(xs)[k * XP + e] = make_float2(v[2 * k], v[2 * k + 1]);
+        }
+        // gradients of the segment's pixels, 32 channels as 8 groups of four per cell
+        const float *gin = c.g + ((size_t)n * c.cout + co0) * c.Ho * c.Wo + y0 * c.Wo + x0;
+        for (int e = lane; e < h * c.segw; e += 32) {
+            const int r = (int)__umulhi((uint32_t)e, by_segw), i = c.segw > 1 ? e - r * c.segw : 0;
+            const int o = (c.segw > 1 ? r : e) * c.Wo + i;
+            const bool ok = i < w;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                float v[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = ok && 4 * k + q < outs ? __ldg(gin + ((4 * k + q) * g_plane + o)) : 0.f;
+                reinterpret_cast<float4 *>(gs)[k * GP + e] = make_float4(v[0], v[1], v[2], v[3]);
+            }
+        }
+        __syncwarp();
+        if (blockIdx.x == 0)
+            for (int e = 0; e < h * c.segw; ++e) bias += gs[((lane >> 2) * GP + e) * 4 + (lane & 3)];
+        for (int r = 0; r < h; ++r) {
+            const float2 *xr = reinterpret_cast<const float2 *>(xs) + p * XP + r * STRIDE * XW;
+            const float4 *gr = reinterpret_cast<const float4 *>(gs) + cg * GP + r * c.segw;
+            auto column = [&](int i, float2 (&v)[3]) {
+#pragma unroll
+                for (int ky = 0; ky < 3; ++ky) v[ky] = xr[ky * XW + i];
+            };
+            auto pixel = [&](int i, const float2 (&k0)[3], const float2 (&k1)[3], const float2 (&k2)[3]) {
+                const float4 gv = gr[i];
+                const float gg[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+                for (int o = 0; o < 4; ++o)
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) {
+                        acc[o][0][3 * ky] = fmaf(gg[o], k0[ky].x, acc[o][0][3 * ky]);
+                        acc[o][1][3 * ky] = fmaf(gg[o], k0[ky].y, acc[o][1][3 * ky]);
+                        acc[o][0][3 * ky + 1] = fmaf(gg[o], k1[ky].x, acc[o][0][3 * ky + 1]);
+                        acc[o][1][3 * ky + 1] = fmaf(gg[o], k1[ky].y, acc[o][1][3 * ky + 1]);
+                        acc[o][0][3 * ky + 2] = fmaf(gg[o], k2[ky].x, acc[o][0][3 * ky + 2]);
+                        acc[o][1][3 * ky + 2] = fmaf(gg[o], k2[ky].y, acc[o][1][3 * ky + 2]);
+                    }
+            };
+            float2 A[3], B[3], C[3];
+            column(0, A);
+            if constexpr (STRIDE == 1) {
+                column(1, B);
+                int i = 0;
+#pragma unroll 1
+                for (; i + 3 <= w; i += 3) {
+                    column(i + 2, C);
+                    pixel(i, A, B, C);
+                    column(i + 3, A);
+                    pixel(i + 1, B, C, A);
+                    column(i + 4, B);
+                    pixel(i + 2, C, A, B);
+                }
+                if (i < w) {
+                    column(i + 2, C);
+                    pixel(i, A, B, C);
+                    if (i + 1 < w) {
+                        column(i + 3, A);
+                        pixel(i + 1, B, C, A);
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int i = 0; i < w; ++i) {
+                    column(2 * i + 1, B);
+                    column(2 * i + 2, C);
+                    pixel(i, A, B, C);
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) A[ky] = C[ky];
+                }
+            }
         }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // sums of warps 4..7, then 2..3, then 1 are added to those of the warps below
+    constexpr int STRIDE_T = 73;  // 72 sums and the bias of a thread
+#pragma unroll 1
+    for (int half = 4; half >= 1; half >>= 1) {
+        __syncthreads();
+        if (warp >= half && warp < 2 * half) {
+            float *d = bw_sm + ((warp - half) * 32 + lane) * STRIDE_T;
 #pragma unroll
-    for (int k = 0; k < COC; ++k)
+            for (int o = 0; o < 4; ++o)
 #pragma unroll
-        for (int t = 0; t < 10; ++t) {
-            float v = acc[k][t];
+                for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) red[warp][k * 10 + t] = v;
+                    for (int t = 0; t < 9; ++t) d[(o * 2 + i) * 9 + t] = acc[o][i][t];
+            d[72] = bias;
         }
-    __syncthreads();
-    for (int e = threadIdx.x; e < NV; e += 256) {
-        float s = 0.f;
+        __syncthreads();
+        if (warp < half) {
+            const float *d = bw_sm + (warp * 32 + lane) * STRIDE_T;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) s += red[w][e];
-        const int k = e / 10, t = e - k * 10, co = co0 + k;
-        if (co >= c.cout) continue;
-        if (t < 9) c.dw[((size_t)co * cin + ci) * 9 + t] = s;
-        else if (ci == 0) c.db[co] = s;
+            for (int o = 0; o < 4; ++o)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) acc[o][i][t] += d[(o * 2 + i) * 9 + t];
+            bias += d[72];
+        }
     }
+    if (warp != 0) return;
+    const size_t nw = (size_t)c.cout * cin * 9;
+    float *out = c.part + blockIdx.z * (nw + c.cout);
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int co = co0 + 4 * cg + o, ci = ci0 + 2 * p + i;
+            if (co < c.cout && ci < cin)
+#pragma unroll
+                for (int t = 0; t < 9; ++t) out[((size_t)co * cin + ci) * 9 + t] = acc[o][i][t];
+        }
+    if (blockIdx.x == 0 && co0 + lane < c.cout) out[nw + co0 + lane] = bias;
+}
+
+// The splits' sums in split order: weights, then biases (contiguous in the gradient vector).
+__global__ void bwd_w_finish_kernel(const float *part, int splits, int n, float *grad)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float v = 0.f;
+    for (int s = 0; s < splits; ++s) v += part[(size_t)s * n + i];
+    grad[i] = v;
 }
 
 // g *= LeakyReLU'(pre-activation), read from the layer output's sign
@@ -791,31 +1053,37 @@ __global__ void act_bwd_kernel(float *g, const float *out, size_t n)
     if (i < n && !(out[i] > 0.f)) g[i] *= kSlope;
 }
 
-// Route dIn of a concatenated input back: ga (+=, summing the 2x2 fine pixels of each
-// coarse pixel when a was upsampled) and gb (+=).
-__global__ void split_grad_kernel(const float *din, int N, int ca, int cb, int up, int Hin, int Win, int Ha, int Wa,
-                                  float *ga, float *gb)
+// Route dIn (the sum of its splits, in split order) of a concatenated input back: ga (+=, summing
+// the 2x2 fine pixels of each coarse pixel when a was upsampled) and gb (+=).
+__global__ void split_grad_kernel(const float *din, int splits, int N, int ca, int cb, int up, int Hin, int Win, int Ha,
+                                  int Wa, float *ga, float *gb)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t na = ga ? (size_t)N * ca * Ha * Wa : 0, nb = gb ? (size_t)N * cb * Hin * Win : 0;
     const int cin = ca + cb;
+    const size_t stride = (size_t)N * cin * Hin * Win;
+    auto at = [&](size_t o) {
+        float v = din[o];
+        for (int k = 1; k < splits; ++k) v += din[k * stride + o];
+        return v;
+    };
     if (i < na) {
         const int X = (int)(i % Wa);
         size_t r = i / Wa;
         const int Y = (int)(r % Ha);
         r /= Ha;
         const int ch = (int)(r % ca), n = (int)(r / ca);
-        const float *src = din + ((size_t)n * cin + ch) * Hin * Win;
+        const size_t src = ((size_t)n * cin + ch) * Hin * Win;
         float s;
         if (up) {
             s = 0.f;
             for (int dy = 0; dy < 2; ++dy)
                 for (int dx = 0; dx < 2; ++dx) {
                     const int y = 2 * Y + dy, x = 2 * X + dx;
-                    if (y < Hin && x < Win) s += src[y * Win + x];
+                    if (y < Hin && x < Win) s += at(src + y * Win + x);
                 }
         } else {
-            s = src[Y * Win + X];
+            s = at(src + Y * Win + X);
         }
         ga[i] += s;
     } else if (i < na + nb) {
@@ -825,17 +1093,36 @@ __global__ void split_grad_kernel(const float *din, int N, int ca, int cb, int u
         const int y = (int)(r % Hin);
         r /= Hin;
         const int ch = (int)(r % cb), n = (int)(r / cb);
-        gb[j] += din[((size_t)n * cin + ca + ch) * Hin * Win + y * Win + x];
+        gb[j] += at(((size_t)n * cin + ca + ch) * Hin * Win + y * Win + x);
+    }
+}
+
+// loss[1] = 1 / sum(mask) (0 for an empty mask), loss[0] = 0.  One block: a fixed order of sums.
+__global__ void __launch_bounds__(1024) mask_kernel(const float *mask, int n, float *loss)
+{
+    __shared__ double red[32];
+    double v = 0;
+    for (int i = threadIdx.x; i < n; i += 1024) v += mask[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        v = 0;
+        for (int w = 0; w < 32; ++w) v += red[w];
+        loss[0] = 0.f;
+        loss[1] = v > 0 ? (float)(1.0 / v) : 0.f;
     }
 }
 
 // Charbonnier loss on the head (downsampled px): sum over masked vectors of
-// sqrt(e^2 + eps^2) - eps per component, times inv_count; its gradient into gpred.
-__global__ void loss_kernel(const float *pred, const float *label, const float *mask, int N, int HW, float inv_count,
-                            float *gpred, float *loss)
+// sqrt(e^2 + eps^2) - eps per component, times loss[1]; its gradient into gpred.
+__global__ void loss_kernel(const float *pred, const float *label, const float *mask, int N, int HW, float *gpred,
+                            float *loss)
 {
     constexpr float eps = 0.01f;
     __shared__ float red[8];
+    const float inv_count = loss[1];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float l = 0.f;
     if (i < N * HW) {
@@ -961,6 +1248,8 @@ struct piv_net {
     size_t t_off[kTensors] = {};
     size_t act_floats = 0, din_floats = 0, part_floats = 0;
     float *act = nullptr, *gact = nullptr, *din = nullptr, *part = nullptr;
+    float *wpart = nullptr;  // splits' sums of the weight gradients (allocated at the first training step)
+    size_t wpart_floats = 0;
     int splits[kLayers] = {};
     float *d_loss = nullptr, *h_loss = nullptr;
     // features scratch
@@ -1052,6 +1341,85 @@ ConvIn conv_in(piv_net *n, const float *base, int i, int N)
     c.Ha = n->lh[la];
     c.Wa = n->lw[la];
     return c;
+}
+
+// output-channel splits of layer i's data gradient: enough CTAs for four per SM, every split at
+// least one group of channels
+int bwd_data_splits(const piv_net *n, int i, int N)
+{
+    const LayerSpec &sp = kSpec[i];
+    if (sp.cout % kBdCo) return 1;
+    const int lin = sp.up ? kLevel[sp.b] : kLevel[sp.a], cin = sp.ca + sp.cb;
+    const int runs = N * n->lh[lin] * ((n->lw[lin] + 7) / 8);
+    const int ctas = ((runs + kBdWarps * kBdRuns - 1) / (kBdWarps * kBdRuns)) * ((cin + 31) / 32);
+    const int chunks = sp.cout / kBdCo, want = std::min(chunks, std::max(1, 4 * 148 / ctas));
+    const int per = (chunks + want - 1) / want;
+    return (chunks + per - 1) / per;  // no empty split
+}
+
+// the weight gradient of layer i: enough splits for two CTAs per SM
+ConvBwdW bwd_w_args(piv_net *n, int i, int N)
+{
+    const LayerSpec &sp = kSpec[i];
+    const int lo = kLevel[i + 1], cin = sp.ca + sp.cb;
+    ConvBwdW c;
+    c.in = conv_in(n, n->act, i, N);
+    c.N = N;
+    c.Ho = n->lh[lo];
+    c.Wo = n->lw[lo];
+    c.stride = sp.stride;
+    c.cout = sp.cout;
+    c.g = n->gact + n->t_off[i + 1];
+    c.part = n->wpart;
+    bwd_w_segments(c);
+    const int tiles = ((cin + 7) / 8) * ((sp.cout + 31) / 32);
+    c.splits = std::max(1, std::min((2 * 148 + tiles - 1) / tiles, (c.segs + 7) / 8));
+    return c;
+}
+
+// the splits' workspaces of the training step, kept by the net (the data gradient's in din)
+int reserve_training(piv_net *n, int N)
+{
+    size_t need = 0, din = n->din_floats;
+    for (int i = 1; i < kLayers; ++i) {
+        const LayerSpec &sp = kSpec[i];
+        const int lin = sp.up ? kLevel[sp.b] : kLevel[sp.a];
+        din = std::max(din, (size_t)bwd_data_splits(n, i, N) * N * (sp.ca + sp.cb) * n->lh[lin] * n->lw[lin]);
+    }
+    if (din > n->din_floats) {
+        cudaFree(n->din);
+        n->din = nullptr;
+        n->din_floats = 0;
+        NCK(cudaMalloc(&n->din, din * sizeof(float)));
+        n->din_floats = din;
+    }
+    for (int i = 0; i < kLayers; ++i) {
+        const size_t nw = (size_t)kSpec[i].cout * ((kSpec[i].ca + kSpec[i].cb) * 9 + 1);
+        need = std::max(need, nw * bwd_w_args(n, i, N).splits);
+    }
+    if (n->wpart && n->wpart_floats >= need) return PIV_OK;
+    cudaFree(n->wpart);
+    n->wpart = nullptr;
+    n->wpart_floats = 0;
+    NCK(cudaMalloc(&n->wpart, need * sizeof(float)));
+    n->wpart_floats = need;
+    NCK(cudaFuncSetAttribute(conv_bwd_w_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwSmem));
+    NCK(cudaFuncSetAttribute(conv_bwd_w_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwSmem));
+    return PIV_OK;
+}
+
+cudaError_t launch_bwd_data(const ConvBwdData &c, int splits, cudaStream_t s)
+{
+    const int runs = c.N * c.Hin * ((c.Win + 7) / 8), per_cta = kBdWarps * kBdRuns;
+    const int chunks = c.cout / kBdCo, per_split = (chunks + splits - 1) / splits * kBdCo;
+    const dim3 grid((runs + per_cta - 1) / per_cta, (c.cin + 31) / 32, splits);
+    auto go = [&](auto kern) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdDataSmem));
+        if (e != cudaSuccess) return e;
+        kern<<<grid, 32 * kBdWarps, sizeof(BwdDataSmem), s>>>(c, per_split);
+        return cudaGetLastError();
+    };
+    return c.stride == 1 ? go(conv_bwd_data_tile_kernel<1>) : go(conv_bwd_data_tile_kernel<2>);
 }
 
 // the forward's weight copy from the FP32 masters (after every change of the weights)
@@ -1253,7 +1621,7 @@ int piv_net_create(uint64_t seed, piv_net **out)
         cudaMalloc(&n->adam_v, off * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&n->wbf, off * sizeof(__nv_bfloat16)) != cudaSuccess ||
         cudaMalloc(&n->wt, n->wt_total * sizeof(__nv_bfloat16)) != cudaSuccess ||
-        cudaMalloc(&n->d_loss, sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&n->d_loss, 2 * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&n->d_status, sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&n->h_loss, sizeof(float)) != cudaSuccess ||
         cudaStreamCreate(&n->stream) != cudaSuccess)  // blocking: ordered after default-stream work
@@ -1287,6 +1655,7 @@ int piv_net_destroy(piv_net *n)
     cudaFree(n->gact);
     cudaFree(n->din);
     cudaFree(n->part);
+    cudaFree(n->wpart);
     cudaFree(n->d_loss);
     cudaFree(n->d_status);
     cudaFree(n->fdown);
@@ -1407,20 +1776,15 @@ int piv_net_loss_grad(piv_net *n, const float *d_in, const float *d_label, const
     cudaSetDevice(n->device);
     int rc = net_reserve(n, N, H, W);
     if (rc) return rc;
+    if ((rc = reserve_training(n, N))) return rc;
     cudaStream_t s = n->stream;
     NCK(net_forward(n, d_in, N, H, W, nullptr, s));
-    // mask count on the device would need a reduction first; the host counts instead
-    std::vector<float> hm((size_t)N * H * W);
-    NCK(cudaMemcpyAsync(hm.data(), d_mask, hm.size() * sizeof(float), cudaMemcpyDeviceToHost, s));
-    NCK(cudaStreamSynchronize(s));
-    double cnt = 0;
-    for (float v : hm) cnt += v;
-    const float inv = cnt > 0 ? (float)(1.0 / cnt) : 0.f;
     NCK(cudaMemsetAsync(n->gact, 0, n->act_floats * sizeof(float), s));
-    NCK(cudaMemsetAsync(n->d_loss, 0, sizeof(float), s));
+    mask_kernel<<<1, 1024, 0, s>>>(d_mask, N * H * W, n->d_loss);
+    NCK(cudaGetLastError());
     const int HW = H * W;
     float *pred = n->act + n->t_off[kTensors - 1], *gpred = n->gact + n->t_off[kTensors - 1];
-    loss_kernel<<<(N * HW + 255) / 256, 256, 0, s>>>(pred, d_label, d_mask, N, HW, inv, gpred, n->d_loss);
+    loss_kernel<<<(N * HW + 255) / 256, 256, 0, s>>>(pred, d_label, d_mask, N, HW, gpred, n->d_loss);
     NCK(cudaGetLastError());
     for (int i = kLayers - 1; i >= 0; --i) {
         const LayerSpec &sp = kSpec[i];
@@ -1433,19 +1797,13 @@ int piv_net_loss_grad(piv_net *n, const float *d_in, const float *d_label, const
             act_bwd_kernel<<<(unsigned)((no + 255) / 256), 256, 0, s>>>(g, o, no);
             NCK(cudaGetLastError());
         }
-        ConvBwdW bw;
-        bw.in = conv_in(n, n->act, i, N);
-        bw.N = N;
-        bw.Ho = Ho;
-        bw.Wo = Wo;
-        bw.stride = sp.stride;
-        bw.cout = sp.cout;
-        bw.g = g;
-        bw.dw = n->grads + n->w_off[i];
-        bw.db = n->grads + n->b_off[i];
-        const int cin = sp.ca + sp.cb;
-        if (sp.cout % 8 == 0) conv_bwd_w_kernel<8><<<dim3(cin, sp.cout / 8), 256, 0, s>>>(bw);
-        else conv_bwd_w_kernel<2><<<dim3(cin, (sp.cout + 1) / 2), 256, 0, s>>>(bw);
+        const ConvBwdW bw = bwd_w_args(n, i, N);
+        const int cin = sp.ca + sp.cb, nw = sp.cout * cin * 9 + sp.cout;
+        const dim3 wgrid((cin + 7) / 8, (sp.cout + 31) / 32, bw.splits);
+        if (sp.stride == 1) conv_bwd_w_kernel<1><<<wgrid, 256, kBwSmem, s>>>(bw);
+        else conv_bwd_w_kernel<2><<<wgrid, 256, kBwSmem, s>>>(bw);
+        NCK(cudaGetLastError());
+        bwd_w_finish_kernel<<<(nw + 255) / 256, 256, 0, s>>>(n->wpart, bw.splits, nw, n->grads + n->w_off[i]);
         NCK(cudaGetLastError());
         if (sp.a == 0 && sp.b < 0) continue;  // the cost volume needs no gradient
         ConvBwdData bd;
@@ -1459,14 +1817,20 @@ int piv_net_loss_grad(piv_net *n, const float *d_in, const float *d_label, const
         bd.cout = sp.cout;
         bd.w = n->wbf + n->w_off[i];
         bd.g = g;
-        bd.din = n->din;
         const int px = bd.Hin * bd.Win;
-        conv_bwd_data_kernel<32><<<dim3((px + 127) / 128, (cin + 31) / 32, N), 128, 0, s>>>(bd);
-        NCK(cudaGetLastError());
+        bd.din = n->din;
+        int splits = 1;
+        if (sp.cout % kBdCo == 0) {
+            splits = bwd_data_splits(n, i, N);
+            NCK(launch_bwd_data(bd, splits, s));
+        } else {
+            conv_bwd_data_kernel<32><<<dim3((px + 127) / 128, (cin + 31) / 32, N), 128, 0, s>>>(bd);
+            NCK(cudaGetLastError());
+        }
         float *ga = sp.a > 0 ? n->gact + n->t_off[sp.a] : nullptr;
         float *gb = sp.b >= 0 ? n->gact + n->t_off[sp.b] : nullptr;
         const size_t tot = (ga ? (size_t)N * sp.ca * bw.in.Ha * bw.in.Wa : 0) + (gb ? (size_t)N * sp.cb * px : 0);
-        split_grad_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(n->din, N, sp.ca, sp.cb, sp.up, bd.Hin,
+        split_grad_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(n->din, splits, N, sp.ca, sp.cb, sp.up, bd.Hin,
                                                                          bd.Win, bw.in.Ha, bw.in.Wa, ga, gb);
         NCK(cudaGetLastError());
     }
