@@ -319,6 +319,7 @@ struct MedianPass {
     float thr;
     int median;        // 0: only copy candidate 0 (Npass_median == 0)
     int *list, *list_n;  // append invalid outputs here when non-NULL (fill work list)
+    int *zero_n;         // set to 0 by a pass before the one that appends
 };
 
 // One pass of organize_median_filter_data + median_validity + Calc_median x4 +
@@ -360,6 +361,49 @@ __device__ __forceinline__ void median_decide(const MedianPass &a, int v, float 
     }
 }
 
+// The register form of one vector (stencils of at most 32 cells).
+__device__ __forceinline__ void median_vector32(const MedianPass &a, int v, float &rx, float &ry, uint8_t &rv)
+{
+    const int Ntm = a.wx * a.wy, centre = (Ntm - 1) / 2;
+    const int vy = v / a.Nx, vx = v - vy * a.Nx;
+    const int hfwx = (a.wx - 1) / 2, hfwy = (a.wy - 1) / 2;
+                const float inf = __int_as_float(0x7f800000);
+                float xs[32], ys[32];
+                int n = 0;
+                int tx = 0, ty = 0;  // stencil column and row of slot t (no division per slot)
+    #pragma unroll
+                for (int t = 0; t < 32; ++t) {
+                    const int x = vx - hfwx + tx, y = vy - hfwy + ty;
+                    const bool inb = (t < Ntm) & (t != centre) & (x >= 0) & (x <= a.Nx - 1) & (y >= 0) & (y <= a.Ny - 1);
+                    bool ok;
+                    float px, py;
+                    median_neighbour(a, inb ? y * a.Nx + x : v, ok, px, py);  // always a valid address
+                    ok = ok & inb;
+                    xs[t] = ok ? px : inf;
+                    ys[t] = ok ? py : inf;
+                    n += ok;
+                    const bool wrap = ++tx == a.wx;
+                    tx = wrap ? 0 : tx;
+                    ty += wrap;
+                }
+                if (n >= a.minN && n >= 1) {
+                    bitonic_sort<32>(xs);
+                    bitonic_sort<32>(ys);
+                    const float mx = median_sorted<32>(xs, n), my = median_sorted<32>(ys, n);
+                    // |x - median| over a sorted x falls, then rises (then +inf): a bitonic
+                    // sequence, which the final merge stage of the network sorts on its own
+    #pragma unroll
+                    for (int q = 0; q < 32; ++q) {
+                        xs[q] = (q < n) ? fabsf(xs[q] - mx) : inf;
+                        ys[q] = (q < n) ? fabsf(ys[q] - my) : inf;
+                    }
+                    bitonic_step<32, 32, 16>(xs);
+                    bitonic_step<32, 32, 16>(ys);
+                    const float dmx = median_sorted<32>(xs, n), dmy = median_sorted<32>(ys, n);
+                    median_decide(a, v, mx, my, dmx, dmy, rx, ry, rv);
+                }
+}
+
 // One pass of organize_median_filter_data + median_validity + Calc_median x4 +
 // Calc_devi x2 + median_filtering (X/xcorr2d_multi_grid.cu:209-296, 1464-1513), one
 // thread per vector.  The medians are order statistics, so how they are found does not
@@ -372,6 +416,7 @@ __global__ void __launch_bounds__(128) median_pass_kernel(const MedianPass a)
     extern __shared__ float sl[];
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     const int Nt = a.Nx * a.Ny;
+    if (a.zero_n && v == 0) *a.zero_n = 0;
     if (v >= Nt) return;
     const int Ntm = a.wx * a.wy;
     float rx = 0.f, ry = 0.f;
@@ -381,46 +426,12 @@ __global__ void __launch_bounds__(128) median_pass_kernel(const MedianPass a)
         ry = a.cdy[(size_t)v * a.Nps];
         rv = a.cvalid[(size_t)v * a.Nps];
     } else {
-        const int vy = v / a.Nx, vx = v - vy * a.Nx;
-        const int hfwx = (a.wx - 1) / 2, hfwy = (a.wy - 1) / 2;
-        const int centre = (Ntm - 1) / 2;
         if constexpr (REG) {
-            const float inf = __int_as_float(0x7f800000);
-            float xs[32], ys[32];
-            int n = 0;
-            int tx = 0, ty = 0;  // stencil column and row of slot t (no division per slot)
-#pragma unroll
-            for (int t = 0; t < 32; ++t) {
-                const int x = vx - hfwx + tx, y = vy - hfwy + ty;
-                const bool inb = (t < Ntm) & (t != centre) & (x >= 0) & (x <= a.Nx - 1) & (y >= 0) & (y <= a.Ny - 1);
-                bool ok;
-                float px, py;
-                median_neighbour(a, inb ? y * a.Nx + x : v, ok, px, py);  // always a valid address
-                ok = ok & inb;
-                xs[t] = ok ? px : inf;
-                ys[t] = ok ? py : inf;
-                n += ok;
-                const bool wrap = ++tx == a.wx;
-                tx = wrap ? 0 : tx;
-                ty += wrap;
-            }
-            if (n >= a.minN && n >= 1) {
-                bitonic_sort<32>(xs);
-                bitonic_sort<32>(ys);
-                const float mx = median_sorted<32>(xs, n), my = median_sorted<32>(ys, n);
-                // |x - median| over a sorted x falls, then rises (then +inf): a bitonic
-                // sequence, which the final merge stage of the network sorts on its own
-#pragma unroll
-                for (int q = 0; q < 32; ++q) {
-                    xs[q] = (q < n) ? fabsf(xs[q] - mx) : inf;
-                    ys[q] = (q < n) ? fabsf(ys[q] - my) : inf;
-                }
-                bitonic_step<32, 32, 16>(xs);
-                bitonic_step<32, 32, 16>(ys);
-                const float dmx = median_sorted<32>(xs, n), dmy = median_sorted<32>(ys, n);
-                median_decide(a, v, mx, my, dmx, dmy, rx, ry, rv);
-            }
+            median_vector32(a, v, rx, ry, rv);
         } else {
+            const int vy = v / a.Nx, vx = v - vy * a.Nx;
+            const int hfwx = (a.wx - 1) / 2, hfwy = (a.wy - 1) / 2;
+            const int centre = (Ntm - 1) / 2;
             // thread-private slices interleaved across threads: element k of thread t at k*blockDim + t
             const int stride = blockDim.x;
             float *xs = sl + threadIdx.x, *ys = sl + (size_t)Ntm * blockDim.x + threadIdx.x;
@@ -455,6 +466,165 @@ __global__ void __launch_bounds__(128) median_pass_kernel(const MedianPass a)
     a.oy[v] = ry;
     a.ov[v] = rv;
     if (a.list && !rv) a.list[atomicAdd(a.list_n, 1)] = v;
+}
+
+// Batcher's merge exchange (Knuth, The Art of Computer Programming 3, algorithm 5.2.2 M):
+// ascending sort of N registers, all indices compile-time.
+template <int N, int P, int Q, int R, int D>
+__device__ __forceinline__ void merge_exchange(float (&a)[N])
+{
+    static_for<0, N - D>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        if constexpr ((i & P) == R) {
+            const float x = a[i], y = a[i + D];
+            a[i] = fminf(x, y);
+            a[i + D] = fmaxf(x, y);
+        }
+    });
+    if constexpr (Q != P) merge_exchange<N, P, Q / 2, P, Q - P>(a);
+}
+template <int N, int P>
+__device__ __forceinline__ void merge_exchange_sort(float (&a)[N])
+{
+    constexpr int T = N <= 32 ? 16 : 0;  // 2^(t - 1), t = ceil(log2 N)
+    static_assert(N > 16 && N <= 32, "one network size class");
+    merge_exchange<N, P, T, 0, P>(a);
+    if constexpr (P > 1) merge_exchange_sort<N, P / 2>(a);
+}
+
+// Median and MAD of one component of a 5x5 neighbourhood that holds an infinity or a NaN
+// (candidates set by the caller).  What fminf and fmaxf make of those depends on the exchanges, so
+// these are median_pass_kernel's, in loops over local memory: rare, and no register is kept for it.
+__device__ __noinline__ float2 median5_nonfinite(const float *src, const uint8_t *flag, int step, int Nx, int Ny,
+                                                 int vx, int vy)
+{
+    const float inf = __int_as_float(0x7f800000);
+    float w[32];
+    int n = 0;
+#pragma unroll 1
+    for (int q = 0; q < 32; ++q) {
+        const int x = vx + q % 5 - 2, y = vy + q / 5 - 2;
+        w[q] = inf;
+        if (q < 25 && q != 12 && x >= 0 && x < Nx && y >= 0 && y < Ny && flag[(size_t)(y * Nx + x) * step]) {
+            w[q] = src[(size_t)(y * Nx + x) * step];
+            ++n;
+        }
+    }
+    float med = 0.f, mad = 0.f;
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+        // the whole network, then its final merge stage
+#pragma unroll 1
+        for (int k = round ? 32 : 2; k <= 32; k *= 2)
+#pragma unroll 1
+            for (int j = k / 2; j > 0; j /= 2)
+#pragma unroll 1
+                for (int i = 0; i < 32; ++i) {
+                    const int l = i ^ j;
+                    if (l < i) continue;
+                    const float lo = fminf(w[i], w[l]), hi = fmaxf(w[i], w[l]);
+                    w[i] = (i & k) ? hi : lo;
+                    w[l] = (i & k) ? lo : hi;
+                }
+        mad = n % 2 ? w[n / 2] : (w[n / 2] + w[n / 2 - 1]) / 2;
+        if (round) break;
+        med = mad;
+#pragma unroll 1
+        for (int q = 0; q < 32; ++q) w[q] = q < n ? fabsf(w[q] - med) : inf;
+    }
+    return make_float2(med, mad);
+}
+
+// The 5x5 stencil (the usual one): two threads per vector, one for each component, which meet by
+// shuffle for the decision.  A component's 24 neighbours are sorted by merge exchange (123
+// exchanges; the 32-slot bitonic network of median_pass_kernel has 240).  With all 24 present,
+// which all but the border vectors have, the median and the MAD need no further sort: the
+// deviations of the lower and the upper half are two sorted lists, whose 12 smallest are
+// min(lower[i], upper[11 - i]).  What bounds it: the latency of the straight-line code on small
+// grids, issue slots on large ones.  Validation of a grid (two median passes, fill, smoothing), one
+// thread per vector with the general network -> this: 21 x 16 vectors 34 -> 23 us, 411 x 274
+// 64 -> 43 us, 384 x 509 98 -> 63 us.  Other stencils keep median_pass_kernel: the exchanges and
+// the two halves of the MAD are laid out for exactly 24 neighbours.
+__global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
+{
+    const int t = blockIdx.x * 128 + threadIdx.x, comp = t & 1, Nt = a.Nx * a.Ny;
+    const bool live = (t >> 1) < Nt;
+    const int v = live ? t >> 1 : Nt - 1;
+    if (a.zero_n && t == 0) *a.zero_n = 0;
+    const int vy = v / a.Nx, vx = v - vy * a.Nx;
+    const float *src = a.ix ? (comp ? a.iy : a.ix) : (comp ? a.cdy : a.cdx);
+    const uint8_t *flag = a.ix ? a.iv : a.cvalid;
+    const int step = a.ix ? 1 : a.Nps;
+    const float inf = __int_as_float(0x7f800000);
+    float s[24];
+    int n = 0;
+    bool odd = false;
+#pragma unroll
+    for (int q = 0; q < 25; ++q) {
+        if (q == 12) continue;  // the centre
+        const int x = vx + q % 5 - 2, y = vy + q / 5 - 2;
+        const bool inb = (unsigned)x < (unsigned)a.Nx && (unsigned)y < (unsigned)a.Ny;
+        const size_t id = (size_t)(inb ? y * a.Nx + x : v) * step;
+        const bool ok = inb && flag[id] != 0;
+        const float f = src[id];
+        s[q < 12 ? q : q - 1] = ok ? f : inf;
+        n += ok;
+        odd |= ok && !(fabsf(f) < inf);
+    }
+    merge_exchange_sort<24, 16>(s);
+    float med, mad;
+    if (odd) {
+        const float2 m = median5_nonfinite(src, flag, step, a.Nx, a.Ny, vx, vy);
+        med = m.x;
+        mad = m.y;
+    } else if (n == 24) {
+        med = (s[12] + s[11]) / 2;
+        float lo = 0.f, hi = inf;
+#pragma unroll
+        for (int i = 0; i < 12; ++i) {
+            const float l = fabsf(s[11 - i] - med), u = fabsf(s[23 - i] - med);  // lower[i], upper[11 - i]
+            lo = fmaxf(lo, fminf(l, u));
+            hi = fminf(hi, fmaxf(l, u));
+        }
+        mad = (hi + lo) / 2;
+    } else {
+        float w[32];
+#pragma unroll
+        for (int q = 0; q < 32; ++q) w[q] = q < 24 ? s[q < 24 ? q : 0] : inf;
+        med = median_sorted<32>(w, n);
+        // |x - median| over a sorted x falls, then rises (then +inf): the network's final merge
+        // stage sorts it
+#pragma unroll
+        for (int q = 0; q < 32; ++q) w[q] = q < n ? fabsf(w[q] - med) : inf;
+        bitonic_step<32, 32, 16>(w);
+        mad = median_sorted<32>(w, n);
+    }
+    // median_filtering's decision (median_decide): the first valid candidate with both residuals
+    // below the threshold
+    const float epsilon = 0.1f;
+    bool found = !(n >= a.minN && n >= 1), ok = false;
+    float r = 0.f;
+    for (int i = 0; i < a.Nps; ++i) {
+        const size_t c = (size_t)v * a.Nps + i;
+        float cand = 0.f;
+        bool pass = false;
+        if (!found && a.cvalid[c]) {
+            cand = comp ? a.cdy[c] : a.cdx[c];
+            pass = __fdiv_rn(fabsf(cand - med), mad + epsilon) < a.thr;
+        }
+        const bool both = __shfl_xor_sync(0xffffffffu, (int)pass, 1) && pass;
+        if (both) {
+            r = cand;
+            ok = found = true;
+        }
+        if (__all_sync(0xffffffffu, found)) break;
+    }
+    if (!live) return;
+    (comp ? a.oy : a.ox)[v] = r;
+    if (comp == 0) {
+        a.ov[v] = ok;
+        if (a.list && !ok) a.list[atomicAdd(a.list_n, 1)] = v;
+    }
 }
 
 // fill_blank_vecfield + fill_blank_vecfield_update repeated until nothing changes
@@ -514,8 +684,9 @@ __global__ void __launch_bounds__(1024) fill_kernel(float *fx, float *fy, uint8_
 
 // organize_smooth_filter_data + smoothing_tophat (X/xcorr2d_multi_grid.cu:399-443):
 // mean over the in-bounds wx x wy stencil, centre included, summed in raster order
-// (the reference sums in atomic-arrival order).
-__global__ void smooth_kernel(const float *ix, const float *iy, float *ox, float *oy, int Nx, int Ny, int wx, int wy)
+// (the reference sums in atomic-arrival order).  The validity is carried along unchanged.
+__global__ void smooth_kernel(const float *ix, const float *iy, const uint8_t *iv, float *ox, float *oy, uint8_t *ov,
+                              int Nx, int Ny, int wx, int wy)
 {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= Nx * Ny) return;
@@ -534,6 +705,7 @@ __global__ void smooth_kernel(const float *ix, const float *iy, float *ox, float
         }
     ox[v] = __fdiv_rn(sx, (float)n);
     oy[v] = __fdiv_rn(sy, (float)n);
+    if (ov != iv) ov[v] = iv[v];
 }
 
 // MedianFilter_Smoothing_p1/p2: median passes (ping-pong), fill in place, smoothing
@@ -548,7 +720,8 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
     const uint8_t *cv = nullptr;
     cudaError_t e = cudaSuccess;
     int *list = a.iffill ? a.list : nullptr;
-    if (list) {
+    // the work list's length starts at 0: an earlier median pass clears it, or a memset
+    if (list && steps_med == 1) {
         e = cudaMemsetAsync(a.list_n, 0, sizeof(int), s);
         if (e != cudaSuccess) return e;
     }
@@ -575,7 +748,10 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         m.median = a.Npass_median > 0;
         m.list = (st == steps_med) ? list : nullptr;
         m.list_n = a.list_n;
-        if (a.wx_med * a.wy_med <= 32) {
+        m.zero_n = (list && st == 1 && steps_med > 1) ? a.list_n : nullptr;
+        if (m.median && a.wx_med == 5 && a.wy_med == 5) {
+            median5_pass_kernel<<<(2 * Nt + 127) / 128, 128, 0, s>>>(m);
+        } else if (a.wx_med * a.wy_med <= 32) {
             median_pass_kernel<true><<<(Nt + tb - 1) / tb, tb, 0, s>>>(m);
         } else {
             const size_t smem = m.median ? (size_t)2 * a.wx_med * a.wy_med * tb * sizeof(float) : 0;
@@ -601,13 +777,8 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         const bool canon = dst_is_canon(st);
         float *ox = canon ? a.fx : a.tx, *oy = canon ? a.fy : a.ty;
         uint8_t *ov = canon ? a.fv : a.tv;
-        smooth_kernel<<<(Nt + 255) / 256, 256, 0, s>>>(cx, cy, ox, oy, a.Nx_vec, a.Ny_vec, a.wx_sm, a.wy_sm);
+        smooth_kernel<<<(Nt + 255) / 256, 256, 0, s>>>(cx, cy, cv, ox, oy, ov, a.Nx_vec, a.Ny_vec, a.wx_sm, a.wy_sm);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        // validity is not changed by smoothing: carry it to the destination buffer
-        if (ov != cv) {
-            e = cudaMemcpyAsync(ov, cv, (size_t)Nt, cudaMemcpyDeviceToDevice, s);
-            if (e != cudaSuccess) return e;
-        }
         cx = ox;
         cy = oy;
         cv = ov;
