@@ -339,18 +339,18 @@ int do_prep(piv_engine *e)
 {
     const piv_params &p = e->p;
     cudaStream_t s = e->stream;
+    const uint8_t *mhe_src[2] = {nullptr, nullptr};
     for (int f = 0; f < 2; ++f) {
         const uint8_t *din = f ? e->d_in2 : e->d_in1;
         uint8_t *dst = f ? e->d_f2 : e->d_f1;
         uint8_t *host = f ? e->h_f2 : e->h_f1;
         if (p.if_mhe == 1) {
-            const uint8_t *src = din;
-            if (!src) {
+            mhe_src[f] = din;
+            if (!din) {
                 uint8_t *stage = f ? e->d_stage2 : e->d_stage1;
                 CK(cudaMemcpyAsync(stage, host, (size_t)p.Nx * p.Ny, cudaMemcpyHostToDevice, s));
-                src = stage;
+                mhe_src[f] = stage;
             }
-            CK(launch_mhe(e->mg, src, p.Nx, e->d_levels, dst, e->pitch, e->mx, e->my, s));
         } else if (din) {
             CK(cudaMemcpy2DAsync(dst + (size_t)e->my * e->pitch + e->mx, e->pitch, din, p.Nx, p.Nx, p.Ny,
                                  cudaMemcpyDeviceToDevice, s));
@@ -359,6 +359,8 @@ int do_prep(piv_engine *e)
                                  cudaMemcpyHostToDevice, s));
         }
     }
+    if (p.if_mhe == 1)
+        CK(launch_mhe_pair(e->mg, mhe_src[0], mhe_src[1], p.Nx, e->d_levels, e->d_f1, e->d_f2, e->pitch, e->mx, e->my, s));
     e->prepared = true;
     return PIV_OK;
 }
@@ -805,7 +807,7 @@ int piv_create(const piv_params *p, piv_engine **out)
         return bail(set_err(e, PIV_ERR_CUDA, "memset failed"));
     if (p->if_mhe == 1) {
         if ((rc = dalloc(e, &e->d_stage1, npix)) || (rc = dalloc(e, &e->d_stage2, npix))) return bail(rc);
-        const size_t nlev = (size_t)(e->mg.maxI + 2) * (e->mg.maxJ + 2) * 256;
+        const size_t nlev = (size_t)2 * (e->mg.maxI + 2) * (e->mg.maxJ + 2) * 256;  // both frames'
         if ((rc = dalloc(e, &e->d_levels, nlev))) return bail(rc);
         if (cudaMemset(e->d_levels, 0, nlev * sizeof(int)) != cudaSuccess)
             return bail(set_err(e, PIV_ERR_CUDA, "memset failed"));
@@ -1452,7 +1454,7 @@ int piv_kernel_launches_per_pair(const piv_engine *e, int *n)
     if (!e || !n) return PIV_ERR_ARG;
     const piv_params &p = e->p;
     auto val = [&](int npm, int nps) { return (npm > 0 ? npm : 1) + 1 /* fill */ + nps; };
-    int k = (p.if_mhe == 1) ? 4 : 0;
+    int k = (p.if_mhe == 1) ? 2 : 0;
     for (int j = 0; j < p.Npass1; ++j)
         k += (j > 0 ? 1 : 0) + e->g.Nsec[0] + val(p.Npass1_median, p.Npass1_smooth);
     if (p.Npass2 > 0) k += 1 + p.Npass2 * (1 + e->g.Nsec[1] + val(p.Npass2_median, p.Npass2_smooth));

@@ -56,8 +56,20 @@ __device__ __forceinline__ bool mhe_words(const uint8_t *p, int pitch, int ws)
 __device__ __forceinline__ int div_small(int q, uint64_t magic) { return (int)(((uint64_t)q * magic) >> 32); }
 __host__ __device__ inline uint64_t div_magic(int d) { return (0x100000000ull + (uint64_t)d - 1) / (uint64_t)d; }
 
-__global__ void __launch_bounds__(256) mhe_hist_kernel(const MheGeom m, const uint8_t *in, int in_pitch, int *levels)
+// One frame, or both of a pair in one launch (blockIdx.y): on small frames, where a launch is a
+// few CTAs, the second frame then costs nothing (enhancement of a pair: 333x251 40 -> 19 us,
+// 1024x1024 21 -> 15, 6600x4400 106 -> 97).
+struct MheFrames {
+    const uint8_t *in[2];
+    uint8_t *out[2];
+    int *levels[2];
+};
+
+template <bool PAIR>
+__global__ void __launch_bounds__(256) mhe_hist_kernel(const MheGeom m, const MheFrames f, int in_pitch)
 {
+    const uint8_t *in = PAIR && blockIdx.y ? f.in[1] : f.in[0];
+    int *levels = PAIR && blockIdx.y ? f.levels[1] : f.levels[0];
     __shared__ int h[kTilesPerCta][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x * kTilesPerCta + warp;
@@ -117,8 +129,8 @@ __global__ void __launch_bounds__(256) mhe_hist_kernel(const MheGeom m, const ui
     for (int b = lane; b < 256; b += 32) dst[b] = hw[b];
 }
 
-__global__ void __launch_bounds__(256) mhe_apply_kernel(const MheGeom m, const uint8_t *in, int in_pitch,
-                                                        const int *levels, uint8_t *out, int out_pitch, int ox, int oy)
+__device__ __forceinline__ void mhe_apply(const MheGeom &m, const uint8_t *in, int in_pitch, const int *levels,
+                                          uint8_t *out, int out_pitch, int ox, int oy)
 {
     __shared__ __align__(16) uint8_t lut_all[kTilesPerCta][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -253,15 +265,44 @@ __global__ void __launch_bounds__(256) mhe_apply_kernel(const MheGeom m, const u
     }
 }
 
+__global__ void __launch_bounds__(256) mhe_apply_kernel(const MheGeom m, const MheFrames f, int in_pitch, int out_pitch,
+                                                        int ox, int oy)
+{
+    mhe_apply(m, f.in[0], in_pitch, f.levels[0], f.out[0], out_pitch, ox, oy);
+}
+// (bounded: the selected pointers would take it from 64 to 79 registers and from 4 to 3 CTAs an SM)
+__global__ void __launch_bounds__(256, 4) mhe_apply_pair_kernel(const MheGeom m, const MheFrames f, int in_pitch,
+                                                                int out_pitch, int ox, int oy)
+{
+    const bool q = blockIdx.y != 0;
+    mhe_apply(m, q ? f.in[1] : f.in[0], in_pitch, q ? f.levels[1] : f.levels[0], q ? f.out[1] : f.out[0], out_pitch,
+              ox, oy);
+}
+
+template <bool PAIR>
+static cudaError_t launch_frames(const MheGeom &m, const MheFrames &f, int in_pitch, int out_pitch, int ox, int oy,
+                                 cudaStream_t s)
+{
+    const dim3 ctas((m.maxI * m.maxJ + kTilesPerCta - 1) / kTilesPerCta, PAIR ? 2 : 1);
+    mhe_hist_kernel<PAIR><<<ctas, 32 * kTilesPerCta, 0, s>>>(m, f, in_pitch);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    if (PAIR) mhe_apply_pair_kernel<<<ctas, 32 * kTilesPerCta, 0, s>>>(m, f, in_pitch, out_pitch, ox, oy);
+    else mhe_apply_kernel<<<ctas, 32 * kTilesPerCta, 0, s>>>(m, f, in_pitch, out_pitch, ox, oy);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_mhe(const MheGeom &m, const uint8_t *in, int in_pitch, int *levels, uint8_t *out, int out_pitch,
                        int ox, int oy, cudaStream_t s)
 {
-    const int ctas = (m.maxI * m.maxJ + kTilesPerCta - 1) / kTilesPerCta;
-    mhe_hist_kernel<<<ctas, 32 * kTilesPerCta, 0, s>>>(m, in, in_pitch, levels);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    mhe_apply_kernel<<<ctas, 32 * kTilesPerCta, 0, s>>>(m, in, in_pitch, levels, out, out_pitch, ox, oy);
-    return cudaGetLastError();
+    return launch_frames<false>(m, MheFrames{{in, in}, {out, out}, {levels, levels}}, in_pitch, out_pitch, ox, oy, s);
+}
+
+cudaError_t launch_mhe_pair(const MheGeom &m, const uint8_t *in1, const uint8_t *in2, int in_pitch, int *levels,
+                            uint8_t *out1, uint8_t *out2, int out_pitch, int ox, int oy, cudaStream_t s)
+{
+    int *second = levels + (size_t)(m.maxI + 2) * (m.maxJ + 2) * 256;
+    return launch_frames<true>(m, MheFrames{{in1, in2}, {out1, out2}, {levels, second}}, in_pitch, out_pitch, ox, oy, s);
 }
 
 }  // namespace piv

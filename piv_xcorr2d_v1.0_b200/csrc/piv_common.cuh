@@ -235,6 +235,10 @@ bool mhe_geometry(int Nx, int Ny, int ws, float thresh, MheGeom &m);
 cudaError_t launch_mhe(const MheGeom &m, const uint8_t *in, int in_pitch, int *levels, uint8_t *out, int out_pitch,
                        int ox, int oy, cudaStream_t s);
 
+// Both frames of a pair in one launch; levels: two such grids, one after the other.
+cudaError_t launch_mhe_pair(const MheGeom &m, const uint8_t *in1, const uint8_t *in2, int in_pitch, int *levels,
+                            uint8_t *out1, uint8_t *out2, int out_pitch, int ox, int oy, cudaStream_t s);
+
 // Status bits written by kernels.
 enum : int { kStatusFillCap = 1, kStatusMmaWait = 2 };
 
