@@ -195,6 +195,10 @@ struct piv_engine {
     };
     ResultSlot results[2];
     int result_seq = 0;
+    // synchronous readback (piv_get_field): two pinned halves that results pass through
+    uint8_t *h_bounce = nullptr;
+    size_t bounce = 0;  // bytes of each half
+    cudaEvent_t ev_bounce[2] = {};
     // learned form (piv_run_pair_learned): its captured graph, keyed by input frames and
     // net; the upsampled prediction kept for the judge; the judge's two numbers
     cudaGraphExec_t learned_exec = nullptr;
@@ -281,7 +285,9 @@ void free_all(piv_engine *e)
     }
     cudaFreeHost(e->h_f1);
     cudaFreeHost(e->h_f2);
-    cudaFreeHost(e->h_status);
+    cudaFreeHost(e->h_status);  // and h_bounce behind it
+    for (auto &ev : e->ev_bounce)
+        if (ev) cudaEventDestroy(ev);
     cudaFree(e->d_stage1);
     cudaFree(e->d_stage2);
     cudaFree(e->d_f1);
@@ -704,6 +710,46 @@ int tune_xcorr(piv_engine *e)
     return rc;
 }
 
+// What follows a wait for the engine stream: the device's error status (its copy is in h_status),
+// then the stage times.
+int after_synchronize(piv_engine *e)
+{
+    if (*e->h_status) {
+        const int st = *e->h_status;
+        CK(cudaMemsetAsync(e->d_status, 0, sizeof(int), e->stream));
+        CK(cudaStreamSynchronize(e->stream));
+        return set_err(e, PIV_ERR_DEVICE, "device status 0x%x (%s)", st,
+                       (st & kStatusMmaWait) ? "tensor-core MMA completion wait timed out"
+                                             : "hole-fill iteration cap reached");
+    }
+    if (e->timing && e->have_times) {
+        cudaEventElapsedTime(&e->stage_ms[0], e->ev[0], e->ev[1]);
+        cudaEventElapsedTime(&e->stage_ms[1], e->ev[1], e->ev[2]);
+        cudaEventElapsedTime(&e->stage_ms[2], e->ev[2], e->ev[3]);
+        cudaEventElapsedTime(&e->stage_ms[4], e->ev[0], e->ev[3]);
+        e->stage_ms[3] = 0.f;
+    }
+    return PIV_OK;
+}
+
+// Grid coordinates of X/xcorr2d_multi_grid.cu:1237-1254 (either pointer may be NULL).
+void grid_coordinates(const GridGeom &g, float *x, float *y)
+{
+    for (int i = 0; x && i < g.Nx_vec; ++i) x[i] = (float)(g.sp_x / 2 + i * g.sp_x);
+    for (int j = 0; j < g.Ny_vec; ++j) {
+        if (x && j > 0) std::memcpy(x + (size_t)j * g.Nx_vec, x, g.Nx_vec * sizeof(float));
+        if (y) std::fill_n(y + (size_t)j * g.Nx_vec, g.Nx_vec, (float)(g.sp_y / 2 + j * g.sp_y));
+    }
+}
+
+// First touch of the caller's pages (fresh ones are mapped on demand), contents unchanged.
+void touch_pages(void *p, size_t bytes)
+{
+    if (!p) return;
+    volatile char *c = static_cast<volatile char *>(p);
+    for (size_t o = 0; o < bytes; o += 4096) c[o] = c[o];
+}
+
 int validate_params(piv_engine *e, const piv_params &p)
 {
     const char *why = nullptr;
@@ -796,10 +842,16 @@ int piv_create(const piv_params *p, piv_engine **out)
     e->pitch = round_up(p->Nx + 2 * e->mx, 128);
     e->rows = p->Ny + 2 * e->my;
     const size_t fbytes = (size_t)e->pitch * e->rows, npix = (size_t)p->Nx * p->Ny;
+    // readback halves: a component of the larger grid, at most 256 KB (pinned memory is slow to get)
+    e->bounce = std::min<size_t>(256 * 1024, ((size_t)std::max(g.Nt_vec[0], g.Nt_vec[1]) * 4 + 4095) & ~(size_t)4095);
     if (cudaHostAlloc((void **)&e->h_f1, npix, cudaHostAllocDefault) != cudaSuccess ||
         cudaHostAlloc((void **)&e->h_f2, npix, cudaHostAllocDefault) != cudaSuccess ||
-        cudaHostAlloc((void **)&e->h_status, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
+        cudaHostAlloc((void **)&e->h_status, 64 + 2 * e->bounce, cudaHostAllocDefault) != cudaSuccess)
         return bail(set_err(e, PIV_ERR_ALLOC, "pinned allocation failed"));
+    e->h_bounce = reinterpret_cast<uint8_t *>(e->h_status) + 64;
+    for (auto &ev : e->ev_bounce)
+        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
+            return bail(set_err(e, PIV_ERR_CUDA, "event creation failed"));
     std::memset(e->h_f1, 0, npix);
     std::memset(e->h_f2, 0, npix);
     if ((rc = dalloc(e, &e->d_f1, fbytes)) || (rc = dalloc(e, &e->d_f2, fbytes))) return bail(rc);
@@ -1185,22 +1237,7 @@ int piv_synchronize(piv_engine *e)
     if (rc) return rc;
     CK(cudaMemcpyAsync(e->h_status, e->d_status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    if (*e->h_status) {
-        const int st = *e->h_status;
-        CK(cudaMemsetAsync(e->d_status, 0, sizeof(int), e->stream));
-        CK(cudaStreamSynchronize(e->stream));
-        return set_err(e, PIV_ERR_DEVICE, "device status 0x%x (%s)", st,
-                       (st & kStatusMmaWait) ? "tensor-core MMA completion wait timed out"
-                                             : "hole-fill iteration cap reached");
-    }
-    if (e->timing && e->have_times) {
-        cudaEventElapsedTime(&e->stage_ms[0], e->ev[0], e->ev[1]);
-        cudaEventElapsedTime(&e->stage_ms[1], e->ev[1], e->ev[2]);
-        cudaEventElapsedTime(&e->stage_ms[2], e->ev[2], e->ev[3]);
-        cudaEventElapsedTime(&e->stage_ms[4], e->ev[0], e->ev[3]);
-        e->stage_ms[3] = 0.f;
-    }
-    return PIV_OK;
+    return after_synchronize(e);
 }
 
 int piv_stage_times(piv_engine *e, float *ms5)
@@ -1219,24 +1256,61 @@ int piv_get_field(piv_engine *e, int sel, float *x, float *y, float *dx, float *
     int rc = check_ready(e, false);
     if (rc) return rc;
     if (sel < 0 || sel > 3) return set_err(e, PIV_ERR_ARG, "selection must be 0..3");
-    if ((rc = piv_synchronize(e))) return rc;
     const int k = sel / 2;
     const bool raw = (sel % 2) == 0;
     const GridState &gs = e->grid[k];
     const size_t Nt = (size_t)gs.gg.Nt_vec, n = raw ? Nt * e->p.Npeak_save : Nt;
-    if (dx) CK(cudaMemcpyAsync(dx, raw ? gs.cdx : gs.fx, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
-    if (dy) CK(cudaMemcpyAsync(dy, raw ? gs.cdy : gs.fy, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
-    if (valid) CK(cudaMemcpyAsync(valid, raw ? gs.cv : gs.fv, n, cudaMemcpyDeviceToHost, e->stream));
-    if (x || y) {
-        for (int j = 0; j < gs.gg.Ny_vec; ++j)
-            for (int i = 0; i < gs.gg.Nx_vec; ++i) {
-                // grid coordinates of X/xcorr2d_multi_grid.cu:1237-1254
-                if (x) x[j * gs.gg.Nx_vec + i] = (float)(gs.gg.sp_x / 2 + i * gs.gg.sp_x);
-                if (y) y[j * gs.gg.Nx_vec + i] = (float)(gs.gg.sp_y / 2 + j * gs.gg.sp_y);
-            }
+    auto known = [](const void *q) {  // pinned, managed or device memory
+        cudaPointerAttributes at;
+        return q && cudaPointerGetAttributes(&at, q) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    };
+    if (known(dx) || known(dy) || known(valid)) {
+        // no host access of ours to what CUDA knows: it takes the copies itself
+        if ((rc = piv_synchronize(e))) return rc;
+        if (dx) CK(cudaMemcpyAsync(dx, raw ? gs.cdx : gs.fx, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+        if (dy) CK(cudaMemcpyAsync(dy, raw ? gs.cdy : gs.fy, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+        if (valid) CK(cudaMemcpyAsync(valid, raw ? gs.cv : gs.fv, n, cudaMemcpyDeviceToHost, e->stream));
+        grid_coordinates(gs.gg, x, y);
+        CK(cudaStreamSynchronize(e->stream));
+        return PIV_OK;
     }
-    CK(cudaStreamSynchronize(e->stream));
-    return PIV_OK;
+    // The results pass through two pinned halves: their copies queue behind the work in flight,
+    // and the host's share (grid coordinates, first touch of the caller's pages) runs beside it.
+    struct Part {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    };
+    std::vector<Part> parts;
+    auto add = [&](void *dst, const void *src, size_t bytes) {
+        if (!dst) return;
+        for (size_t o = 0; o < bytes; o += e->bounce)
+            parts.push_back({(char *)dst + o, (const char *)src + o, std::min(e->bounce, bytes - o)});
+    };
+    add(dx, raw ? gs.cdx : gs.fx, n * sizeof(float));
+    add(dy, raw ? gs.cdy : gs.fy, n * sizeof(float));
+    add(valid, raw ? gs.cv : gs.fv, n);
+    CK(cudaMemcpyAsync(e->h_status, e->d_status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    auto queue = [&](size_t i) {
+        CK(cudaMemcpyAsync(e->h_bounce + (i & 1) * e->bounce, parts[i].src, parts[i].bytes, cudaMemcpyDeviceToHost, e->stream));
+        CK(cudaEventRecord(e->ev_bounce[i & 1], e->stream));
+        return PIV_OK;
+    };
+    for (size_t i = 0; i < parts.size() && i < 2; ++i)
+        if ((rc = queue(i))) return rc;
+    for (const Part &p : parts) touch_pages(p.dst, p.bytes);
+    grid_coordinates(gs.gg, x, y);
+    if (parts.empty()) CK(cudaStreamSynchronize(e->stream));
+    for (size_t i = 0; i < parts.size(); ++i) {
+        CK(cudaEventSynchronize(e->ev_bounce[i & 1]));
+        if (i == 0 && *e->h_status) {
+            CK(cudaStreamSynchronize(e->stream));  // the second half's copy is in flight
+            break;
+        }
+        std::memcpy(parts[i].dst, e->h_bounce + (i & 1) * e->bounce, parts[i].bytes);
+        if (i + 2 < parts.size() && (rc = queue(i + 2))) return rc;
+    }
+    return after_synchronize(e);
 }
 
 int piv_field_async(piv_engine *e, int sel, int *ticket)
@@ -1289,25 +1363,22 @@ int piv_field_wait(piv_engine *e, int ticket, float *x, float *y, float *dx, flo
     piv_engine::ResultSlot &r = e->results[ticket & 1];
     if (!r.pending || r.seq != (ticket >> 1)) return set_err(e, PIV_ERR_STATE, "no pending readback with this ticket");
     cudaSetDevice(e->device);
+    const GridState &gs = e->grid[r.sel / 2];
+    const size_t Nt = (size_t)gs.gg.Nt_vec, n = (r.sel % 2 == 0) ? Nt * e->p.Npeak_save : Nt;
+    // beside the work in flight: grid coordinates, first touch of the caller's pages
+    touch_pages(dx, n * sizeof(float));
+    touch_pages(dy, n * sizeof(float));
+    touch_pages(valid, n);
+    grid_coordinates(gs.gg, x, y);
     CK(cudaEventSynchronize(r.ev));
     r.pending = false;
     if (*r.status)
         return set_err(e, PIV_ERR_DEVICE, "device status 0x%x (%s)", *r.status,
                        (*r.status & kStatusMmaWait) ? "tensor-core MMA completion wait timed out"
                                                     : "hole-fill iteration cap reached");
-    const GridState &gs = e->grid[r.sel / 2];
-    const size_t Nt = (size_t)gs.gg.Nt_vec, n = (r.sel % 2 == 0) ? Nt * e->p.Npeak_save : Nt;
     if (dx) std::memcpy(dx, r.dx, n * sizeof(float));
     if (dy) std::memcpy(dy, r.dy, n * sizeof(float));
     if (valid) std::memcpy(valid, r.valid, n);
-    if (x || y) {
-        for (int j = 0; j < gs.gg.Ny_vec; ++j)
-            for (int i = 0; i < gs.gg.Nx_vec; ++i) {
-                // grid coordinates of X/xcorr2d_multi_grid.cu:1237-1254
-                if (x) x[j * gs.gg.Nx_vec + i] = (float)(gs.gg.sp_x / 2 + i * gs.gg.sp_x);
-                if (y) y[j * gs.gg.Nx_vec + i] = (float)(gs.gg.sp_y / 2 + j * gs.gg.sp_y);
-            }
-    }
     return PIV_OK;
 }
 
