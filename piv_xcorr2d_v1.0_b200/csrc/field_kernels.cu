@@ -5,6 +5,7 @@
 // field with a 3-cell edge-replicated border) is not materialised: every read of the
 // extended field at (m, n) reads the field at (clamp(m-3), clamp(n-3)), which is the
 // same value.
+#include "fft_reg.cuh"
 #include "piv_common.cuh"
 
 namespace piv {
@@ -19,142 +20,300 @@ __device__ __forceinline__ float ext_field(const float *f, int Nx, int Ny, int m
 
 // ------------------------------------------------------------------------------
 // Kernel_Window_Deformation_2d (X/xcorr2d_multi_grid.cu:608-652, launched at :1300
-// and :1624).  Each thread produces 4 consecutive pixels of one row of the
-// [Ny_aug][Nx_aug] deformed image and stores them as one float4.  The arithmetic is
-// written exactly as the reference writes it.  Frame-2 taps outside the padded
-// frame read 0 (the reference reads its zero padding there, or out of bounds).
+// and :1624): bilinear displacement of every pixel of the [Ny_aug][Nx_aug] extent, then
+// bilinear interpolation of frame 2 there.  Every product and sum is rounded as the
+// reference's, written out because neighbouring pixels share packed FP32 instructions.
+// Frame-2 taps outside the padded frame read 0 (the reference reads its zero padding there,
+// or out of bounds).
+//
+// What bounds it: instructions, the conversion pipe and the latency of the byte gathers.  Against
+// one scalar pixel after another (83 instructions and 7 conversions a pixel, every tap's bounds
+// checked):
+//   - floor(x) in integer and float form comes from one addition: x + 1.5 * 2^23 rounded down
+//     holds it in its low bits (|x| < 2^22), so only the bytes go through the conversion pipe;
+//   - a cell's displacements lie between its corners', so one test of the corners clears a whole
+//     run of pixels; runs near the frame's border, and displacements that are no small numbers,
+//     take deform_any.
+// Two mappings, 6600x4400 at spacing 16: 82 us before, 70 by deform_cell8_kernel, 82 by
+// deform_kernel; 4096x2160 at 12: 47 -> 28 us by deform_kernel; 2048x1536 at 4 (20): 21.5 -> 13
+// (22.5 -> 12).
 // ------------------------------------------------------------------------------
-// One output pixel of Kernel_Window_Deformation_2d given the 8 field values of its cell.
-__device__ __forceinline__ float deform_pixel(const DeformArgs &a, int idx, int Y, float a_x, float a_y, float u1,
-                                              float u2, float u3, float u4, float v1, float v2, float v3, float v4,
-                                              int col_off, int row_off)
+constexpr int kDeformRows = 32, kDeformThreads = 128, kDeformMinCtas = 600;
+constexpr int kDeformFar = 1 << 21;  // positions that the addition of 1.5 * 2^23 splits, with room to spare
+
+// One pixel at (px, py): taps may lie outside the frame, and the position may be any number.
+__device__ __noinline__ float deform_any(const Frame8 &f, float px, float py, int col_off, int row_off)
 {
-    float ce1 = (1 - a_x) * (1 - a_y);
-    float ce2 = a_x * (1 - a_y);
-    float ce3 = (1 - a_x) * a_y;
-    float ce4 = a_x * a_y;
-    a_x = (float)idx + ce1 * u1 + ce2 * u2 + ce3 * u3 + ce4 * u4;
-    a_y = (float)Y + ce1 * v1 + ce2 * v2 + ce3 * v3 + ce4 * v4;
-    int i_x = (int)floorf(a_x);
-    int i_y = (int)floorf(a_y);
-    a_x = a_x - (float)i_x;
-    a_y = a_y - (float)i_y;
-    // aug_ex column i_x + hfws_x holds image column i_x - Nx_left -> padded-frame column
-    const int c0 = i_x + col_off, r0 = i_y + row_off;
+    const int i_x = (int)floorf(px), i_y = (int)floorf(py);
+    const float a_x = __fsub_rn(px, (float)i_x), a_y = __fsub_rn(py, (float)i_y);
     float p[4];
-    if (c0 >= 0 && c0 + 1 < a.f2.cols && r0 >= 0 && r0 + 1 < a.f2.rows) {
-        // all four taps inside the padded frame (the common case): no per-tap checks
-        const uint8_t *q = a.f2.base + (size_t)r0 * a.f2.pitch + c0;
-        p[0] = (float)__ldg(q);
-        p[1] = (float)__ldg(q + 1);
-        p[2] = (float)__ldg(q + a.f2.pitch);
-        p[3] = (float)__ldg(q + a.f2.pitch + 1);
-    } else {
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int c = c0 + (t & 1), r = r0 + (t >> 1);
-            p[t] = (c >= 0 && c < a.f2.cols && r >= 0 && r < a.f2.rows)
-                       ? (float)__ldg(a.f2.base + (size_t)r * a.f2.pitch + c)
-                       : 0.f;
-        }
+    for (int t = 0; t < 4; ++t) {
+        const int c = i_x + col_off + (t & 1), r = i_y + row_off + (t >> 1);
+        p[t] = (c >= 0 && c < f.cols && r >= 0 && r < f.rows) ? (float)__ldg(f.base + (size_t)r * f.pitch + c) : 0.f;
     }
-    ce1 = (1 - a_x) * (1 - a_y);
-    ce2 = a_x * (1 - a_y);
-    ce3 = (1 - a_x) * a_y;
-    ce4 = a_x * a_y;
-    return ce1 * p[0] + ce2 * p[1] + ce3 * p[2] + ce4 * p[3];
+    const float b_x = __fsub_rn(1.f, a_x), b_y = __fsub_rn(1.f, a_y);
+    const float s = __fmaf_rn(__fmul_rn(b_x, b_y), p[0], __fmul_rn(__fmul_rn(a_x, b_y), p[1]));
+    return __fmaf_rn(__fmul_rn(a_x, a_y), p[3], __fmaf_rn(__fmul_rn(b_x, a_y), p[2], s));
 }
 
-// (v - st) / sp as the reference writes it; for a power-of-two spacing the reciprocal
-// is exact, and multiplying by it gives the identical correctly rounded quotient.
-template <bool POW2>
-__device__ __forceinline__ float cell_coord(float v, float st, float sp, float inv_sp)
+// Any spacing: a thread makes two neighbouring columns and walks down `rows` rows.  What depends on
+// the column alone (the cell's column, the weights, the divisions by the spacing) is done once, the
+// rows' weights come from a table, and the field is read where the rows enter the next cell.
+template <class Off>
+__global__ void __launch_bounds__(kDeformThreads) deform_kernel(const __grid_constant__ DeformArgs a, const int rows)
 {
-    if constexpr (POW2) return (v - st) * inv_sp;
-    else return (v - st) / sp;
+    __shared__ float4 s_row[kDeformRows];  // (a_y, a_y, 1 - a_y, 1 - a_y)
+    const int X0 = (blockIdx.x * kDeformThreads + threadIdx.x) * 2;
+    const int Y0 = blockIdx.y * rows, Y1 = min(Y0 + rows, a.Ny_aug);
+    const int st_x = a.hfws_x - a.sp_x * 3, st_y = a.hfws_y - a.sp_y * 3;  // origin of the extended field
+    auto cell = [](int v, int st, int sp) { return ((float)v - (float)st) / (float)sp; };
+    if (threadIdx.x < rows) {
+        const float y = cell(Y0 + threadIdx.x, st_y, a.sp_y), a_y = y - floorf(y);
+        s_row[threadIdx.x] = make_float4(a_y, a_y, 1.f - a_y, 1.f - a_y);
+    }
+    __syncthreads();
+    if (X0 >= a.Nx_aug) return;
+    const int col_off = a.f2.mx - a.Nx_left, row_off = a.f2.my - a.Ny_left;
+    const float xa = cell(X0, st_x, a.sp_x), xb = cell(X0 + 1, st_x, a.sp_x);
+    const float fa = floorf(xa), fb = floorf(xb);
+    const float2 one = make_float2(1.f, 1.f), minus = make_float2(-1.f, -1.f);
+    const float2 a_x = make_float2(xa - fa, xb - fb), b_x = __fadd2_rn(one, make_float2(-a_x.x, -a_x.y));
+    // the clamped field columns of both pixels' cells
+    const int ca = clampi((int)fa - 3, 0, a.Nx_vec - 1), ca1 = clampi((int)fa - 2, 0, a.Nx_vec - 1);
+    const int cb = clampi((int)fb - 3, 0, a.Nx_vec - 1), cb1 = clampi((int)fb - 2, 0, a.Nx_vec - 1);
+    float2 u1, u2, u3, u4, v1, v2, v3, v4;
+    auto field_row = [&](int n, float2 &ul, float2 &ur, float2 &vl, float2 &vr) {
+        const size_t o = (size_t)clampi(n - 3, 0, a.Ny_vec - 1) * a.Nx_vec;
+        const float *u = a.fx + o, *v = a.fy + o;
+        ul = make_float2(__ldg(u + ca), __ldg(u + cb));
+        ur = make_float2(__ldg(u + ca1), __ldg(u + cb1));
+        vl = make_float2(__ldg(v + ca), __ldg(v + cb));
+        vr = make_float2(__ldg(v + ca1), __ldg(v + cb1));
+    };
+    const float2 X = make_float2((float)X0, (float)(X0 + 1));
+    const float kMagic = 12582912.f;  // 1.5 * 2^23
+    const float2 magic = make_float2(kMagic, kMagic), unmagic = make_float2(-kMagic, -kMagic);
+    const int pitch = a.f2.pitch;
+    const uint8_t *base = a.f2.base, *base1 = base + pitch;
+    const Off k0 = (Off)(row_off - 0x4B400000) * (Off)pitch + (Off)(col_off - 0x4B400000);
+    const bool both = X0 + 1 < a.Nx_aug;
+    float *dst = a.out + (size_t)Y0 * a.out_pitch + X0;
+
+    auto position = [&](int Y, float2 fy, float2 &px, float2 &py) {
+        const float4 w = s_row[Y - Y0];
+        const float2 a_y = make_float2(w.x, w.y), b_y = make_float2(w.z, w.w);
+        const float2 c1 = __fmul2_rn(b_x, b_y), c2 = __fmul2_rn(a_x, b_y);
+        const float2 c3 = __fmul2_rn(b_x, a_y), c4 = __fmul2_rn(a_x, a_y);
+        px = __ffma2_rn(c4, u4, __ffma2_rn(c3, u3, __ffma2_rn(c2, u2, __ffma2_rn(c1, u1, X))));
+        py = __ffma2_rn(c4, v4, __ffma2_rn(c3, v3, __ffma2_rn(c2, v2, __ffma2_rn(c1, v1, fy))));
+    };
+    auto store = [&](float2 res) {
+        if (both) *reinterpret_cast<float2 *>(dst) = res;
+        else *dst = res.x;
+        dst += a.out_pitch;
+    };
+    // N rows whose taps all lie in the frame: all loads before their use
+    auto run = [&](auto nc, int Y, float2 fy) {
+        constexpr int N = decltype(nc)::value;
+        float2 px[N], py[N], tx[N], ty[N];
+        unsigned char p[N][8];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            position(Y + i, fy, px[i], py[i]);
+            fy = __fadd2_rn(fy, one);
+            tx[i] = __fadd2_rd(px[i], magic);
+            ty[i] = __fadd2_rd(py[i], magic);
+            const Off oa = (Off)__float_as_int(ty[i].x) * (Off)pitch + ((Off)__float_as_int(tx[i].x) + k0);
+            const Off ob = (Off)__float_as_int(ty[i].y) * (Off)pitch + ((Off)__float_as_int(tx[i].y) + k0);
+            const uint8_t *pa = base + oa, *pb = base + ob, *pa1 = base1 + oa, *pb1 = base1 + ob;
+            p[i][0] = __ldg(pa);
+            p[i][1] = __ldg(pb);
+            p[i][2] = __ldg(pa + 1);
+            p[i][3] = __ldg(pb + 1);
+            p[i][4] = __ldg(pa1);
+            p[i][5] = __ldg(pb1);
+            p[i][6] = __ldg(pa1 + 1);
+            p[i][7] = __ldg(pb1 + 1);
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            auto tap = [&](int t) { return make_float2((float)p[i][2 * t], (float)p[i][2 * t + 1]); };
+            const float2 ax = __ffma2_rn(__fadd2_rn(tx[i], unmagic), minus, px[i]);
+            const float2 ay = __ffma2_rn(__fadd2_rn(ty[i], unmagic), minus, py[i]);
+            const float2 bx = __ffma2_rn(ax, minus, one), by = __ffma2_rn(ay, minus, one);
+            const float2 s = __ffma2_rn(__fmul2_rn(bx, by), tap(0), __fmul2_rn(__fmul2_rn(ax, by), tap(1)));
+            store(__ffma2_rn(__fmul2_rn(ax, ay), tap(3), __ffma2_rn(__fmul2_rn(bx, ay), tap(2), s)));
+        }
+    };
+
+    int Y = Y0, i_y = (int)floorf(cell(Y0, st_y, a.sp_y));
+    float2 fy = make_float2((float)Y0, (float)Y0);
+    field_row(i_y, u3, u4, v3, v4);
+    while (true) {
+        u1 = u3;
+        u2 = u4;
+        v1 = v3;
+        v2 = v4;
+        field_row(i_y + 1, u3, u4, v3, v4);
+        // the rows of this cell; their displacements lie between the corners'
+        const int end = min(Y1, st_y + (i_y + 1) * a.sp_y);
+        auto lowest = [](float2 p, float2 q, float2 r, float2 s) {
+            return fminf(fminf(fminf(p.x, p.y), fminf(q.x, q.y)), fminf(fminf(r.x, r.y), fminf(s.x, s.y)));
+        };
+        auto highest = [](float2 p, float2 q, float2 r, float2 s) {
+            return fmaxf(fmaxf(fmaxf(p.x, p.y), fmaxf(q.x, q.y)), fmaxf(fmaxf(r.x, r.y), fmaxf(s.x, s.y)));
+        };
+        // a NaN corner makes sum NaN
+        const float2 uv = __fadd2_rn(__fadd2_rn(__fadd2_rn(u1, u2), __fadd2_rn(u3, u4)),
+                                     __fadd2_rn(__fadd2_rn(v1, v2), __fadd2_rn(v3, v4)));
+        const float sum = uv.x + uv.y;
+        const bool inside = X.x + lowest(u1, u2, u3, u4) >= (float)(1 - col_off) &&
+                            X.y + highest(u1, u2, u3, u4) < (float)(min(a.f2.cols, kDeformFar) - 3 - col_off) &&
+                            fy.x + lowest(v1, v2, v3, v4) >= (float)(1 - row_off) &&
+                            (float)end + highest(v1, v2, v3, v4) < (float)(min(a.f2.rows, kDeformFar) - 3 - row_off) &&
+                            sum == sum;
+        if (inside) {
+            for (; Y + 2 <= end; Y += 2) {
+                run(std::integral_constant<int, 2>{}, Y, fy);
+                fy = __fadd2_rn(fy, make_float2((float)(2), (float)(2)));
+            }
+            for (; Y < end; ++Y) {
+                run(std::integral_constant<int, 1>{}, Y, fy);
+                fy = __fadd2_rn(fy, one);
+            }
+        } else {
+#pragma unroll 1
+            for (; Y < end; ++Y) {
+                float2 px, py;
+                position(Y, fy, px, py);
+                const float left = deform_any(a.f2, px.x, py.x, col_off, row_off);
+                store(make_float2(left, deform_any(a.f2, px.y, py.y, col_off, row_off)));
+                fy = __fadd2_rn(fy, one);
+            }
+        }
+        if (Y >= Y1) break;
+        ++i_y;
+    }
 }
 
-// Each thread writes 8 consecutive pixels of one row (two float4 stores).  When the
-// vector spacing and the field origin are multiples of 8 (the `cell8` launches), the 8
-// pixels lie in one cell of the field, so its 8 values are loaded once.  Bounded to 6
-// blocks per SM (40 registers; the byte gathers want the warps: 88 -> 82 us at the
-// 6600x4400 workload, against no change at 5 blocks and the unbounded 54 registers' 4).
-template <bool CELL8, bool POW2>
-__global__ void __launch_bounds__(256, 6) deform_kernel(const DeformArgs a)
+// Spacings and origins that are multiples of 8: runs of 8 pixels of a row share a cell, whose 8
+// values are loaded once for a thread's one run.  Bounded to 40 registers (6 CTAs per SM): the
+// gathers' latency wants the warps (4 CTAs 76 us, 6 CTAs 70, unbounded 93 at 6600x4400).
+template <class Off, bool POW2>
+__global__ void __launch_bounds__(256, 6) deform_cell8_kernel(const __grid_constant__ DeformArgs a)
 {
     const int X0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
     const int Y = blockIdx.y;
-    if (X0 >= a.Nx_aug || Y >= a.Ny_aug) return;
-    const float x_st_vec = (float)(a.hfws_x - a.sp_x * 3), y_st_vec = (float)(a.hfws_y - a.sp_y * 3);
-    const float vsx = (float)a.sp_x, vsy = (float)a.sp_y;
-    const float ivx = 1.0f / vsx, ivy = 1.0f / vsy;
+    if (X0 >= a.Nx_aug) return;
+    const float x_st = (float)(a.hfws_x - a.sp_x * 3), y_st = (float)(a.hfws_y - a.sp_y * 3);
     const int col_off = a.f2.mx - a.Nx_left, row_off = a.f2.my - a.Ny_left;
-
-    float a_y = cell_coord<POW2>((float)Y, y_st_vec, vsy, ivy);
-    const int i_y = (int)floorf(a_y);
-    a_y = a_y - (float)i_y;
-
-    float res[8];
-    if (CELL8) {
-        const int i_x = (int)floorf(cell_coord<POW2>((float)X0, x_st_vec, vsx, ivx));
-        const float u1 = ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x, i_y);
-        const float u2 = ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x + 1, i_y);
-        const float u3 = ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x, i_y + 1);
-        const float u4 = ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x + 1, i_y + 1);
-        const float v1 = ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x, i_y);
-        const float v2 = ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x + 1, i_y);
-        const float v3 = ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x, i_y + 1);
-        const float v4 = ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x + 1, i_y + 1);
+    // a power of two's reciprocal is exact, and so is the quotient by it
+    const float ix = 1.f / (float)a.sp_x, iy = 1.f / (float)a.sp_y;
+    auto cell = [](float v, float st, float sp, float inv) { return POW2 ? (v - st) * inv : (v - st) / sp; };
+    const float y = cell((float)Y, y_st, (float)a.sp_y, iy), fy = floorf(y), a_y = y - fy, b_y = 1.f - a_y;
+    const float fx = floorf(cell((float)X0, x_st, (float)a.sp_x, ix));
+    const int i_x = (int)fx, i_y = (int)fy;
+    auto field = [&](const float *f, int m, int n) { return ext_field(f, a.Nx_vec, a.Ny_vec, i_x + m, i_y + n); };
+    const float u1 = field(a.fx, 0, 0), u2 = field(a.fx, 1, 0), u3 = field(a.fx, 0, 1), u4 = field(a.fx, 1, 1);
+    const float v1 = field(a.fy, 0, 0), v2 = field(a.fy, 1, 0), v3 = field(a.fy, 0, 1), v4 = field(a.fy, 1, 1);
+    const float2 one = make_float2(1.f, 1.f), minus = make_float2(-1.f, -1.f);
+    const float kMagic = 12582912.f;  // 1.5 * 2^23
+    const float2 magic = make_float2(kMagic, kMagic), unmagic = make_float2(-kMagic, -kMagic);
+    float2 px[4], py[4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int idx = X0 + q;
-            float a_x = cell_coord<POW2>((float)idx, x_st_vec, vsx, ivx);
-            a_x = a_x - (float)i_x;
-            res[q] = deform_pixel(a, idx, Y, a_x, a_y, u1, u2, u3, u4, v1, v2, v3, v4, col_off, row_off);
+    for (int q = 0; q < 4; ++q) {
+        const float2 X = make_float2((float)(X0 + 2 * q), (float)(X0 + 2 * q + 1));
+        const float xa = cell(X.x, x_st, (float)a.sp_x, ix), xb = cell(X.y, x_st, (float)a.sp_x, ix);
+        const float2 a_x = make_float2(xa - fx, xb - fx);
+        const float2 b_x = __ffma2_rn(a_x, minus, one);
+        const float2 c1 = vmul(b_x, b_y), c2 = vmul(a_x, b_y), c3 = vmul(b_x, a_y), c4 = vmul(a_x, a_y);
+        px[q] = vfma(c4, u4, vfma(c3, u3, vfma(c2, u2, vfma(c1, u1, X))));
+        py[q] = vfma(c4, v4, vfma(c3, v3, vfma(c2, v2, vfma(c1, v1, make_float2((float)Y, (float)Y)))));
+    }
+    // the displacements lie between the corners' (a NaN corner makes the sum NaN)
+    const float sum = ((u1 + u2) + (u3 + u4)) + ((v1 + v2) + (v3 + v4));
+    const bool inside = (float)X0 + fminf(fminf(u1, u2), fminf(u3, u4)) >= (float)(1 - col_off) &&
+                        (float)X0 + fmaxf(fmaxf(u1, u2), fmaxf(u3, u4)) <
+                            (float)(min(a.f2.cols, kDeformFar) - 10 - col_off) &&
+                        (float)Y + fminf(fminf(v1, v2), fminf(v3, v4)) >= (float)(1 - row_off) &&
+                        (float)Y + fmaxf(fmaxf(v1, v2), fmaxf(v3, v4)) <
+                            (float)(min(a.f2.rows, kDeformFar) - 3 - row_off) &&
+                        sum == sum;
+    float2 res[4];
+    if (inside) {
+        const int pitch = a.f2.pitch;
+        const uint8_t *base = a.f2.base, *base1 = base + pitch;
+        const Off k0 = (Off)(row_off - 0x4B400000) * (Off)pitch + (Off)(col_off - 0x4B400000);
+        unsigned char p[4][8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float2 tx = __fadd2_rd(px[q], magic), ty = __fadd2_rd(py[q], magic);
+            const Off oa = (Off)__float_as_int(ty.x) * (Off)pitch + ((Off)__float_as_int(tx.x) + k0);
+            const Off ob = (Off)__float_as_int(ty.y) * (Off)pitch + ((Off)__float_as_int(tx.y) + k0);
+            const uint8_t *pa = base + oa, *pb = base + ob, *pa1 = base1 + oa, *pb1 = base1 + ob;
+            p[q][0] = __ldg(pa);
+            p[q][1] = __ldg(pb);
+            p[q][2] = __ldg(pa + 1);
+            p[q][3] = __ldg(pb + 1);
+            p[q][4] = __ldg(pa1);
+            p[q][5] = __ldg(pb1);
+            p[q][6] = __ldg(pa1 + 1);
+            p[q][7] = __ldg(pb1 + 1);
+            // the fractions
+            px[q] = __ffma2_rn(__fadd2_rn(tx, unmagic), minus, px[q]);
+            py[q] = __ffma2_rn(__fadd2_rn(ty, unmagic), minus, py[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            auto tap = [&](int t) { return make_float2((float)p[q][2 * t], (float)p[q][2 * t + 1]); };
+            const float2 ax = px[q], ay = py[q], bx = __ffma2_rn(ax, minus, one), by = __ffma2_rn(ay, minus, one);
+            const float2 s = __ffma2_rn(__fmul2_rn(bx, by), tap(0), __fmul2_rn(__fmul2_rn(ax, by), tap(1)));
+            res[q] = __ffma2_rn(__fmul2_rn(ax, ay), tap(3), __ffma2_rn(__fmul2_rn(bx, ay), tap(2), s));
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int idx = X0 + q;
-            float a_x = cell_coord<POW2>((float)idx, x_st_vec, vsx, ivx);
-            const int i_x = (int)floorf(a_x);
-            a_x = a_x - (float)i_x;
-            res[q] = deform_pixel(a, idx, Y, a_x, a_y, ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x, i_y),
-                                  ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x + 1, i_y),
-                                  ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x, i_y + 1),
-                                  ext_field(a.fx, a.Nx_vec, a.Ny_vec, i_x + 1, i_y + 1),
-                                  ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x, i_y),
-                                  ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x + 1, i_y),
-                                  ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x, i_y + 1),
-                                  ext_field(a.fy, a.Nx_vec, a.Ny_vec, i_x + 1, i_y + 1), col_off, row_off);
-        }
+        for (int q = 0; q < 4; ++q)
+            res[q] = make_float2(deform_any(a.f2, px[q].x, py[q].x, col_off, row_off),
+                                 deform_any(a.f2, px[q].y, py[q].y, col_off, row_off));
     }
     float *dst = a.out + (size_t)Y * a.out_pitch + X0;
     if (X0 + 7 < a.Nx_aug) {
-        reinterpret_cast<float4 *>(dst)[0] = make_float4(res[0], res[1], res[2], res[3]);
-        reinterpret_cast<float4 *>(dst)[1] = make_float4(res[4], res[5], res[6], res[7]);
+        reinterpret_cast<float4 *>(dst)[0] = make_float4(res[0].x, res[0].y, res[1].x, res[1].y);
+        reinterpret_cast<float4 *>(dst)[1] = make_float4(res[2].x, res[2].y, res[3].x, res[3].y);
     } else {
-        for (int q = 0; q < 8 && X0 + q < a.Nx_aug; ++q) dst[q] = res[q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (X0 + 2 * q < a.Nx_aug) dst[2 * q] = res[q].x;
+            if (X0 + 2 * q + 1 < a.Nx_aug) dst[2 * q + 1] = res[q].y;
+        }
     }
+}
+
+template <class Off>
+void launch_deform_as(const DeformArgs &a, cudaStream_t s)
+{
+    // the cell edges x_st + m * sp are multiples of 8; the cell index is then exact for every pixel
+    // of a run (its float quotient is exact for these small integers)
+    const int x_st = a.hfws_x - a.sp_x * 3;
+    if (a.sp_x % 8 == 0 && x_st % 8 == 0) {
+        const dim3 grid(((a.Nx_aug + 7) / 8 + 255) / 256, a.Ny_aug);
+        const bool pow2 = (a.sp_x & (a.sp_x - 1)) == 0 && (a.sp_y & (a.sp_y - 1)) == 0;
+        if (pow2) deform_cell8_kernel<Off, true><<<grid, 256, 0, s>>>(a);
+        else deform_cell8_kernel<Off, false><<<grid, 256, 0, s>>>(a);
+        return;
+    }
+    // rows per thread: as many as leave four CTAs per SM (a CTA's start is 2 to 3 us of latency)
+    const int gx = (a.Nx_aug + 2 * kDeformThreads - 1) / (2 * kDeformThreads);
+    int rows = kDeformRows;
+    while (rows > 2 && gx * ((a.Ny_aug + rows - 1) / rows) < kDeformMinCtas) rows /= 2;
+    deform_kernel<Off><<<dim3(gx, (a.Ny_aug + rows - 1) / rows), kDeformThreads, 0, s>>>(a, rows);
 }
 
 cudaError_t launch_deform(const DeformArgs &a, cudaStream_t s)
 {
-    dim3 block(256);
-    dim3 grid(((a.Nx_aug + 7) / 8 + 255) / 256, a.Ny_aug);
-    // the 8-pixel runs X0..X0+7 (X0 % 8 == 0) share a field cell when the cell edges
-    // x_st + m*sp are multiples of 8; the cell index is then exact for every pixel of
-    // the run (its float quotient is exact for these small integers)
-    const int x_st = a.hfws_x - a.sp_x * 3;
-    const bool cell8 = (a.sp_x % 8 == 0) && (((x_st % 8) + 8) % 8 == 0);
-    const bool pow2 = a.sp_x > 0 && a.sp_y > 0 && (a.sp_x & (a.sp_x - 1)) == 0 && (a.sp_y & (a.sp_y - 1)) == 0;
-    if (cell8) {
-        if (pow2) deform_kernel<true, true><<<grid, block, 0, s>>>(a);
-        else deform_kernel<true, false><<<grid, block, 0, s>>>(a);
-    } else {
-        if (pow2) deform_kernel<false, true><<<grid, block, 0, s>>>(a);
-        else deform_kernel<false, false><<<grid, block, 0, s>>>(a);
-    }
+    if ((uint64_t)a.f2.pitch * a.f2.rows <= UINT32_MAX) launch_deform_as<uint32_t>(a, s);
+    else launch_deform_as<uint64_t>(a, s);
     return cudaGetLastError();
 }
 
