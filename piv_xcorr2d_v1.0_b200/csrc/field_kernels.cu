@@ -15,7 +15,7 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // Extended-field value at ext index (m, n) of a field with Nx x Ny vectors.
 __device__ __forceinline__ float ext_field(const float *f, int Nx, int Ny, int m, int n)
 {
-    return __ldg(f + clampi(n - 3, 0, Ny - 1) * Nx + clampi(m - 3, 0, Nx - 1));
+    return *(f + clampi(n - 3, 0, Ny - 1) * Nx + clampi(m - 3, 0, Nx - 1));
 }
 
 // ------------------------------------------------------------------------------
@@ -50,7 +50,7 @@ __device__ __noinline__ float deform_any(const Frame8 &f, float px, float py, in
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
         const int c = i_x + col_off + (t & 1), r = i_y + row_off + (t >> 1);
-        p[t] = (c >= 0 && c < f.cols && r >= 0 && r < f.rows) ? (float)__ldg(f.base + (size_t)r * f.pitch + c) : 0.f;
+        p[t] = (c >= 0 && c < f.cols && r >= 0 && r < f.rows) ? (float)*(f.base + (size_t)r * f.pitch + c) : 0.f;
     }
     const float b_x = __fsub_rn(1.f, a_x), b_y = __fsub_rn(1.f, a_y);
     const float s = __fmaf_rn(__fmul_rn(b_x, b_y), p[0], __fmul_rn(__fmul_rn(a_x, b_y), p[1]));
@@ -82,14 +82,15 @@ __global__ void __launch_bounds__(kDeformThreads) deform_kernel(const __grid_con
     // the clamped field columns of both pixels' cells
     const int ca = clampi((int)fa - 3, 0, a.Nx_vec - 1), ca1 = clampi((int)fa - 2, 0, a.Nx_vec - 1);
     const int cb = clampi((int)fb - 3, 0, a.Nx_vec - 1), cb1 = clampi((int)fb - 2, 0, a.Nx_vec - 1);
+    chain_start();
     float2 u1, u2, u3, u4, v1, v2, v3, v4;
     auto field_row = [&](int n, float2 &ul, float2 &ur, float2 &vl, float2 &vr) {
         const size_t o = (size_t)clampi(n - 3, 0, a.Ny_vec - 1) * a.Nx_vec;
         const float *u = a.fx + o, *v = a.fy + o;
-        ul = make_float2(__ldg(u + ca), __ldg(u + cb));
-        ur = make_float2(__ldg(u + ca1), __ldg(u + cb1));
-        vl = make_float2(__ldg(v + ca), __ldg(v + cb));
-        vr = make_float2(__ldg(v + ca1), __ldg(v + cb1));
+        ul = make_float2(*(u + ca), *(u + cb));
+        ur = make_float2(*(u + ca1), *(u + cb1));
+        vl = make_float2(*(v + ca), *(v + cb));
+        vr = make_float2(*(v + ca1), *(v + cb1));
     };
     const float2 X = make_float2((float)X0, (float)(X0 + 1));
     const float kMagic = 12582912.f;  // 1.5 * 2^23
@@ -127,14 +128,14 @@ __global__ void __launch_bounds__(kDeformThreads) deform_kernel(const __grid_con
             const Off oa = (Off)__float_as_int(ty[i].x) * (Off)pitch + ((Off)__float_as_int(tx[i].x) + k0);
             const Off ob = (Off)__float_as_int(ty[i].y) * (Off)pitch + ((Off)__float_as_int(tx[i].y) + k0);
             const uint8_t *pa = base + oa, *pb = base + ob, *pa1 = base1 + oa, *pb1 = base1 + ob;
-            p[i][0] = __ldg(pa);
-            p[i][1] = __ldg(pb);
-            p[i][2] = __ldg(pa + 1);
-            p[i][3] = __ldg(pb + 1);
-            p[i][4] = __ldg(pa1);
-            p[i][5] = __ldg(pb1);
-            p[i][6] = __ldg(pa1 + 1);
-            p[i][7] = __ldg(pb1 + 1);
+            p[i][0] = *(pa);
+            p[i][1] = *(pb);
+            p[i][2] = *(pa + 1);
+            p[i][3] = *(pb + 1);
+            p[i][4] = *(pa1);
+            p[i][5] = *(pb1);
+            p[i][6] = *(pa1 + 1);
+            p[i][7] = *(pb1 + 1);
         }
 #pragma unroll
         for (int i = 0; i < N; ++i) {
@@ -203,6 +204,7 @@ __global__ void __launch_bounds__(kDeformThreads) deform_kernel(const __grid_con
 template <class Off, bool POW2>
 __global__ void __launch_bounds__(256, 6) deform_cell8_kernel(const __grid_constant__ DeformArgs a)
 {
+    chain_start();
     const int X0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
     const int Y = blockIdx.y;
     if (X0 >= a.Nx_aug) return;
@@ -252,14 +254,14 @@ __global__ void __launch_bounds__(256, 6) deform_cell8_kernel(const __grid_const
             const Off oa = (Off)__float_as_int(ty.x) * (Off)pitch + ((Off)__float_as_int(tx.x) + k0);
             const Off ob = (Off)__float_as_int(ty.y) * (Off)pitch + ((Off)__float_as_int(tx.y) + k0);
             const uint8_t *pa = base + oa, *pb = base + ob, *pa1 = base1 + oa, *pb1 = base1 + ob;
-            p[q][0] = __ldg(pa);
-            p[q][1] = __ldg(pb);
-            p[q][2] = __ldg(pa + 1);
-            p[q][3] = __ldg(pb + 1);
-            p[q][4] = __ldg(pa1);
-            p[q][5] = __ldg(pb1);
-            p[q][6] = __ldg(pa1 + 1);
-            p[q][7] = __ldg(pb1 + 1);
+            p[q][0] = *(pa);
+            p[q][1] = *(pb);
+            p[q][2] = *(pa + 1);
+            p[q][3] = *(pb + 1);
+            p[q][4] = *(pa1);
+            p[q][5] = *(pb1);
+            p[q][6] = *(pa1 + 1);
+            p[q][7] = *(pb1 + 1);
             // the fractions
             px[q] = __ffma2_rn(__fadd2_rn(tx, unmagic), minus, px[q]);
             py[q] = __ffma2_rn(__fadd2_rn(ty, unmagic), minus, py[q]);
@@ -299,15 +301,15 @@ void launch_deform_as(const DeformArgs &a, cudaStream_t s)
     if (a.sp_x % 8 == 0 && x_st % 8 == 0) {
         const dim3 grid(((a.Nx_aug + 7) / 8 + 255) / 256, a.Ny_aug);
         const bool pow2 = (a.sp_x & (a.sp_x - 1)) == 0 && (a.sp_y & (a.sp_y - 1)) == 0;
-        if (pow2) deform_cell8_kernel<Off, true><<<grid, 256, 0, s>>>(a);
-        else deform_cell8_kernel<Off, false><<<grid, 256, 0, s>>>(a);
+        if (pow2) launch_chained(deform_cell8_kernel<Off, true>, grid, dim3(256), 0, s, a);
+        else launch_chained(deform_cell8_kernel<Off, false>, grid, dim3(256), 0, s, a);
         return;
     }
     // rows per thread: as many as leave four CTAs per SM (a CTA's start is 2 to 3 us of latency)
     const int gx = (a.Nx_aug + 2 * kDeformThreads - 1) / (2 * kDeformThreads);
     int rows = kDeformRows;
     while (rows > 2 && gx * ((a.Ny_aug + rows - 1) / rows) < kDeformMinCtas) rows /= 2;
-    deform_kernel<Off><<<dim3(gx, (a.Ny_aug + rows - 1) / rows), kDeformThreads, 0, s>>>(a, rows);
+    launch_chained(deform_kernel<Off>, dim3(gx, (a.Ny_aug + rows - 1) / rows), dim3(kDeformThreads), 0, s, a, rows);
 }
 
 cudaError_t launch_deform(const DeformArgs &a, cudaStream_t s)
@@ -353,6 +355,7 @@ cudaError_t launch_pattern(uint8_t *u8, float *f32, int pitch, int cols, int row
 // ------------------------------------------------------------------------------
 __global__ void upsample_kernel(const UpsampleArgs a)
 {
+    chain_start();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= a.Nx2 * a.Ny2) return;
     const float x_st_vec1 = (float)(a.sp_x1 / 2 - 3 * a.sp_x1), y_st_vec1 = (float)(a.sp_y1 / 2 - 3 * a.sp_y1);
@@ -382,7 +385,7 @@ __global__ void upsample_kernel(const UpsampleArgs a)
 cudaError_t launch_upsample(const UpsampleArgs &a, cudaStream_t s)
 {
     const int n = a.Nx2 * a.Ny2;
-    upsample_kernel<<<(n + 255) / 256, 256, 0, s>>>(a);
+    launch_chained(upsample_kernel, dim3((n + 255) / 256), dim3(256), 0, s, a);
     return cudaGetLastError();
 }
 
@@ -572,6 +575,7 @@ __device__ __forceinline__ void median_vector32(const MedianPass &a, int v, floa
 template <bool REG>
 __global__ void __launch_bounds__(128) median_pass_kernel(const MedianPass a)
 {
+    chain_start();
     extern __shared__ float sl[];
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     const int Nt = a.Nx * a.Ny;
@@ -706,6 +710,7 @@ __device__ __noinline__ float2 median5_nonfinite(const float *src, const uint8_t
 // the two halves of the MAD are laid out for exactly 24 neighbours.
 __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
 {
+    chain_start();
     const int t = blockIdx.x * 128 + threadIdx.x, comp = t & 1, Nt = a.Nx * a.Ny;
     const bool live = (t >> 1) < Nt;
     const int v = live ? t >> 1 : Nt - 1;
@@ -798,6 +803,7 @@ __global__ void __launch_bounds__(1024) fill_kernel(float *fx, float *fy, uint8_
                                                     const int *list, const int *list_n, int *status,
                                                     int cap_override)
 {
+    chain_start();
     __shared__ int s_cnt[2];
     const int n = *list_n;
     const int cap = cap_override > 0 ? cap_override : Nx + Ny + 2;
@@ -847,6 +853,7 @@ __global__ void __launch_bounds__(1024) fill_kernel(float *fx, float *fy, uint8_
 __global__ void smooth_kernel(const float *ix, const float *iy, const uint8_t *iv, float *ox, float *oy, uint8_t *ov,
                               int Nx, int Ny, int wx, int wy)
 {
+    chain_start();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= Nx * Ny) return;
     const int vy = v / Nx, vx = v - vy * Nx;
@@ -909,9 +916,9 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         m.list_n = a.list_n;
         m.zero_n = (list && st == 1 && steps_med > 1) ? a.list_n : nullptr;
         if (m.median && a.wx_med == 5 && a.wy_med == 5) {
-            median5_pass_kernel<<<(2 * Nt + 127) / 128, 128, 0, s>>>(m);
+            launch_chained(median5_pass_kernel, dim3((2 * Nt + 127) / 128), dim3(128), 0, s, m);
         } else if (a.wx_med * a.wy_med <= 32) {
-            median_pass_kernel<true><<<(Nt + tb - 1) / tb, tb, 0, s>>>(m);
+            launch_chained(median_pass_kernel<true>, dim3((Nt + tb - 1) / tb), dim3(tb), 0, s, m);
         } else {
             const size_t smem = m.median ? (size_t)2 * a.wx_med * a.wy_med * tb * sizeof(float) : 0;
             if (smem > 48 * 1024) {
@@ -919,7 +926,7 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
                                          (int)smem);
                 if (e != cudaSuccess) return e;
             }
-            median_pass_kernel<false><<<(Nt + tb - 1) / tb, tb, smem, s>>>(m);
+            launch_chained(median_pass_kernel<false>, dim3((Nt + tb - 1) / tb), dim3(tb), smem, s, m);
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         cx = m.ox;
@@ -927,7 +934,7 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         cv = m.ov;
     }
     if (a.iffill) {
-        fill_kernel<<<1, 1024, 0, s>>>(const_cast<float *>(cx), const_cast<float *>(cy), const_cast<uint8_t *>(cv),
+        launch_chained(fill_kernel, dim3(1), dim3(1024), 0, s, const_cast<float *>(cx), const_cast<float *>(cy), const_cast<uint8_t *>(cv),
                                        a.Nx_vec, a.Ny_vec, a.list, a.list_n, a.status, a.fill_cap);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -936,7 +943,7 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         const bool canon = dst_is_canon(st);
         float *ox = canon ? a.fx : a.tx, *oy = canon ? a.fy : a.ty;
         uint8_t *ov = canon ? a.fv : a.tv;
-        smooth_kernel<<<(Nt + 255) / 256, 256, 0, s>>>(cx, cy, cv, ox, oy, ov, a.Nx_vec, a.Ny_vec, a.wx_sm, a.wy_sm);
+        launch_chained(smooth_kernel, dim3((Nt + 255) / 256), dim3(256), 0, s, cx, cy, cv, ox, oy, ov, a.Nx_vec, a.Ny_vec, a.wx_sm, a.wy_sm);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         cx = ox;
         cy = oy;

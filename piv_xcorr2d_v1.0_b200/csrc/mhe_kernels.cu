@@ -68,6 +68,7 @@ struct MheFrames {
 template <bool PAIR>
 __global__ void __launch_bounds__(256) mhe_hist_kernel(const MheGeom m, const MheFrames f, int in_pitch)
 {
+    chain_start();
     const uint8_t *in = PAIR && blockIdx.y ? f.in[1] : f.in[0];
     int *levels = PAIR && blockIdx.y ? f.levels[1] : f.levels[0];
     __shared__ int h[kTilesPerCta][256];
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(256) mhe_hist_kernel(const MheGeom m, const Mh
                 v[k] = 0;
                 if (q < nw) {
                     const int r = div_small(q, mg), c = q - r * wpr;
-                    v[k] = __ldg(reinterpret_cast<const uint32_t *>(src + (size_t)r * in_pitch) + c);
+                    v[k] = *(reinterpret_cast<const uint32_t *>(src + (size_t)r * in_pitch) + c);
                 }
             }
 #pragma unroll
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(256) mhe_hist_kernel(const MheGeom m, const Mh
                 v[k] = -1;
                 if (p < npx) {
                     const int r = div_small(p, mg), c = p - r * m.ws;
-                    v[k] = __ldg(src + (size_t)r * in_pitch + c);
+                    v[k] = *(src + (size_t)r * in_pitch + c);
                 }
             }
 #pragma unroll
@@ -154,10 +155,11 @@ __device__ __forceinline__ void mhe_apply(const MheGeom &m, const uint8_t *in, i
             pre[k] = 0;
             if (q < nw) {
                 const int r = div_small(q, mgw), cc = q - r * wpr;
-                pre[k] = __ldg(reinterpret_cast<const uint32_t *>(src + (size_t)r * in_pitch) + cc);
+                pre[k] = *(reinterpret_cast<const uint32_t *>(src + (size_t)r * in_pitch) + cc);
             }
         }
     }
+    chain_start();  // the pixels above are from before the histogram kernel, which had waited for them
     // CreateTransfer_kernel: 3x3 tile neighbourhood of the zero-ringed grid; this lane
     // owns bins [8 lane, 8 lane + 8)
     int tr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -166,7 +168,7 @@ __device__ __forceinline__ void mhe_apply(const MheGeom &m, const uint8_t *in, i
 #pragma unroll
         for (int dx = -1; dx <= 1; ++dx) {
             const int4 *h = reinterpret_cast<const int4 *>(levels + (size_t)(c + dy * W + dx) * 256 + 8 * lane);
-            const int4 u = __ldg(h), w = __ldg(h + 1);
+            const int4 u = *(h), w = *(h + 1);
             tr[0] += u.x;
             tr[1] += u.y;
             tr[2] += u.z;
@@ -224,7 +226,7 @@ __device__ __forceinline__ void mhe_apply(const MheGeom &m, const uint8_t *in, i
                     w[k] = 0;
                     if (q < nw) {
                         const int r = div_small(q, mgw), cc = q - r * wpr;
-                        w[k] = __ldg(reinterpret_cast<const uint32_t *>(src + (size_t)r * in_pitch) + cc);
+                        w[k] = *(reinterpret_cast<const uint32_t *>(src + (size_t)r * in_pitch) + cc);
                     }
                 }
             }
@@ -250,7 +252,7 @@ __device__ __forceinline__ void mhe_apply(const MheGeom &m, const uint8_t *in, i
                 px[k] = 0;
                 if (p < npx) {
                     const int r = div_small(p, mgp), cc = p - r * m.ws;
-                    px[k] = __ldg(src + (size_t)r * in_pitch + cc);
+                    px[k] = *(src + (size_t)r * in_pitch + cc);
                 }
             }
 #pragma unroll
@@ -284,11 +286,11 @@ static cudaError_t launch_frames(const MheGeom &m, const MheFrames &f, int in_pi
                                  cudaStream_t s)
 {
     const dim3 ctas((m.maxI * m.maxJ + kTilesPerCta - 1) / kTilesPerCta, PAIR ? 2 : 1);
-    mhe_hist_kernel<PAIR><<<ctas, 32 * kTilesPerCta, 0, s>>>(m, f, in_pitch);
+    launch_chained(mhe_hist_kernel<PAIR>, ctas, dim3(32 * kTilesPerCta), 0, s, m, f, in_pitch);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (PAIR) mhe_apply_pair_kernel<<<ctas, 32 * kTilesPerCta, 0, s>>>(m, f, in_pitch, out_pitch, ox, oy);
-    else mhe_apply_kernel<<<ctas, 32 * kTilesPerCta, 0, s>>>(m, f, in_pitch, out_pitch, ox, oy);
+    if (PAIR) launch_chained(mhe_apply_pair_kernel, ctas, dim3(32 * kTilesPerCta), 0, s, m, f, in_pitch, out_pitch, ox, oy);
+    else launch_chained(mhe_apply_kernel, ctas, dim3(32 * kTilesPerCta), 0, s, m, f, in_pitch, out_pitch, ox, oy);
     return cudaGetLastError();
 }
 

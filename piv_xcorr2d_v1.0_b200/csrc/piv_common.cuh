@@ -13,6 +13,33 @@
 
 namespace piv {
 
+// Programmatic dependent launch.  The kernels of a pair follow one another in one stream, and on
+// small frames each takes a few microseconds, a good part of them the launch itself.  A kernel
+// launched with launch_chained may be set up while the one before it still runs; it starts with
+// chain_start(), which waits until everything before it in the stream is complete and its writes
+// are visible, and then lets the next one be set up.  So at most one kernel waits at a time, and
+// nothing is read or written before its turn.
+__device__ __forceinline__ void chain_start()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute chained = {};
+    chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    chained.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &chained;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------------------------
 // Compile-time twiddle factors.  exp(-2*pi*i*a/n) is generated in FP64 at compile
 // time: exact octant reduction of the rational angle a/n, then a Taylor series on

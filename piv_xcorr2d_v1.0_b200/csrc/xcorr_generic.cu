@@ -373,6 +373,7 @@ template <bool DEF, bool ANY, bool SMEM>
 __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel(const XcorrArgs a,
                                                                                  const GenericPlan pl, float2 *gplane)
 {
+    chain_start();
     const GridGeom &g = a.g;
     const int nx = g.ws_x, ny = g.ws_y, N = nx * ny, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     extern __shared__ __align__(16) unsigned char gsm[];
@@ -636,7 +637,7 @@ cudaError_t launch_xcorr_generic(const XcorrArgs &a, bool deformed, float2 *work
         // keeps running under the attribute set last
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
         if (e != cudaSuccess) return;
-        kern<<<ctas, kGenThreads, smem, s>>>(a, pl, workspace);
+        launch_chained(kern, dim3(ctas), dim3(kGenThreads), smem, s, a, pl, workspace);
         e = cudaGetLastError();
     };
     auto pick = [&](auto any, auto in_smem) {

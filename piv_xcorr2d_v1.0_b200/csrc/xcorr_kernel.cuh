@@ -646,6 +646,7 @@ constexpr int xcorr_min_ctas()
 template <int WSX, int WSY, int B, int NT, int K, bool DEF>
 __global__ void __launch_bounds__(NT, (xcorr_min_ctas<WSX, WSY, B, NT>())) xcorr_peak_kernel(const XcorrArgs a)
 {
+    chain_start();
     constexpr int VB = 1;
     const unsigned blk = blockIdx.x;
 #include "xcorr_body.inc"
@@ -657,6 +658,7 @@ __global__ void __launch_bounds__(NT, (xcorr_min_ctas<WSX, WSY, B, NT>())) xcorr
 template <int WSX, int WSY, int NT, int K, bool DEF>
 __global__ void __launch_bounds__(NT, (xcorr_min_ctas<WSX, WSY, 4, NT>())) xcorr_block_kernel(const XcorrArgs a)
 {
+    chain_start();
     constexpr int B = 4, VB = 2;
     const unsigned blk = blockIdx.x;
 #include "xcorr_body.inc"
@@ -694,12 +696,14 @@ struct PairShared {
 template <int NW, int K, bool DEF>
 __global__ void __launch_bounds__(32 * NW, 16 / NW) xcorr_pair_kernel(const XcorrArgs a)
 {
+    chain_start();
     const unsigned blk = blockIdx.x;
 #include "xcorr_pair_body.inc"
 }
 template <int NW, int K, bool DEF>
 __global__ void __launch_bounds__(32 * NW, 16 / NW) xcorr_pair_batch_kernel(const __grid_constant__ XcorrBatch b)
 {
+    chain_start();
     const int lo = batch_pair(b, blockIdx.x);
     const XcorrArgs &a = b.pairs[lo];
     const unsigned blk = blockIdx.x - b.first[lo];
@@ -717,6 +721,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) xcorr_pair_batch_kernel(cons
 template <int WSX, int WSY, int B, int NT, int K, bool DEF>
 __global__ void __launch_bounds__(NT, (xcorr_min_ctas<WSX, WSY, B, NT>())) xcorr_batch_kernel(const __grid_constant__ XcorrBatch b)
 {
+    chain_start();
     const int lo = batch_pair(b, blockIdx.x);
     const XcorrArgs &a = b.pairs[lo];
     const unsigned blk = blockIdx.x - b.first[lo];
@@ -738,7 +743,7 @@ cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t 
     auto go = [&](auto kern) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        kern<<<grid, NT, smem, s>>>(a);
+        launch_chained(kern, grid, dim3(NT), smem, s, a);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -767,7 +772,7 @@ cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, int K, cudaStr
     auto go = [&](auto kern) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        kern<<<grid, NT, smem, s>>>(a);
+        launch_chained(kern, grid, dim3(NT), smem, s, a);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -791,7 +796,7 @@ cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaSt
     auto go = [&](auto kern) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        kern<<<b.items, NT, smem, s>>>(b);
+        launch_chained(kern, dim3(b.items), dim3(NT), smem, s, b);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -815,7 +820,7 @@ cudaError_t launch_pair(const XcorrArgs &a, bool deformed, int K, cudaStream_t s
         const size_t smem = (size_t)NW * cells * sizeof(float4);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        kern<<<(pairs + NW - 1) / NW, 32 * NW, smem, s>>>(a);
+        launch_chained(kern, dim3((pairs + NW - 1) / NW), dim3(32 * NW), smem, s, a);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -837,7 +842,7 @@ cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, int K, cudaStr
         const size_t smem = (size_t)NW * cells * sizeof(float4);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        kern<<<b.items, 32 * NW, smem, s>>>(b);
+        launch_chained(kern, dim3(b.items), dim3(32 * NW), smem, s, b);
         e = cudaGetLastError();
     };
     if (K <= 4) {
