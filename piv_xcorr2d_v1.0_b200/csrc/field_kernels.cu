@@ -934,8 +934,9 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         cv = m.ov;
     }
     if (a.iffill) {
-        launch_chained(fill_kernel, dim3(1), dim3(1024), 0, s, const_cast<float *>(cx), const_cast<float *>(cy), const_cast<uint8_t *>(cv),
-                                       a.Nx_vec, a.Ny_vec, a.list, a.list_n, a.status, a.fill_cap);
+        launch_chained(fill_kernel, dim3(1), dim3(1024), 0, s, const_cast<float *>(cx), const_cast<float *>(cy),
+                       const_cast<uint8_t *>(cv),
+                       a.Nx_vec, a.Ny_vec, a.list, a.list_n, a.status, a.fill_cap);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     for (int k = 0; k < a.Npass_smooth; ++k) {
@@ -943,7 +944,8 @@ cudaError_t launch_validate(const ValidateArgs &a, cudaStream_t s)
         const bool canon = dst_is_canon(st);
         float *ox = canon ? a.fx : a.tx, *oy = canon ? a.fy : a.ty;
         uint8_t *ov = canon ? a.fv : a.tv;
-        launch_chained(smooth_kernel, dim3((Nt + 255) / 256), dim3(256), 0, s, cx, cy, cv, ox, oy, ov, a.Nx_vec, a.Ny_vec, a.wx_sm, a.wy_sm);
+        launch_chained(smooth_kernel, dim3((Nt + 255) / 256), dim3(256), 0, s, cx, cy, cv, ox, oy, ov, a.Nx_vec,
+                       a.Ny_vec, a.wx_sm, a.wy_sm);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         cx = ox;
         cy = oy;
