@@ -637,7 +637,7 @@ cudaError_t launch_xcorr_generic(const XcorrArgs &a, bool deformed, float2 *work
         // keeps running under the attribute set last
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
         if (e != cudaSuccess) return;
-        launch_chained(kern, dim3(ctas), dim3(kGenThreads), smem, s, a, pl, workspace);
+        kern<<<ctas, kGenThreads, smem, s>>>(a, pl, workspace);
         e = cudaGetLastError();
     };
     auto pick = [&](auto any, auto in_smem) {

@@ -1,4 +1,4 @@
-// xcorr_kernel.cu -- the fused correlation + peak kernel (FP32 SIMT path).
+// xcorr_kernel.cuh -- the fused correlation + peak kernel (FP32 SIMT path).
 //
 // One launch replaces, for a section of windows, the reference's
 //   organize_data_fft2d_multi(_deformed)  X/xcorr2d_multi_grid.cu:497, 654
@@ -17,8 +17,8 @@
 // Per CTA: a batch of B windows (B even).  Every transform is one thread's, on packed FP32
 // pairs (fft_reg.cuh); shared memory is laid out so that each phase's pairs come in with one
 // 16-byte load per two elements (Plane below).  Data flow:
-//   P1  row task (window, row): gather frame-1 and frame-2 rows straight from HBM,
-//       pack z = f1 + i*f2, row FFT in registers, store.
+//   P1  the windows' pixel rows are staged in shared memory by cp.async (Raw below); row task
+//       (window, row): read both frames' rows, pack z = f1 + i*f2, row FFT in registers, store.
 //   P2  column task: column FFT in registers -> Z = FFT2(f1) + i*FFT2(f2).
 //   P3  column task (window pair, column): the cross spectrum conj(F1)*F2 follows
 //       from Z(k) and Z(-k) as  C = Im(Z(k)Z(-k))/2 + i(|Z(-k)|^2 - |Z(k)|^2)/4;
@@ -743,7 +743,7 @@ cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t 
     auto go = [&](auto kern) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        launch_chained(kern, grid, dim3(NT), smem, s, a);
+        kern<<<grid, NT, smem, s>>>(a);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -772,7 +772,7 @@ cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, int K, cudaStr
     auto go = [&](auto kern) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        launch_chained(kern, grid, dim3(NT), smem, s, a);
+        kern<<<grid, NT, smem, s>>>(a);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -796,7 +796,7 @@ cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaSt
     auto go = [&](auto kern) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        launch_chained(kern, dim3(b.items), dim3(NT), smem, s, b);
+        kern<<<b.items, NT, smem, s>>>(b);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -820,7 +820,7 @@ cudaError_t launch_pair(const XcorrArgs &a, bool deformed, int K, cudaStream_t s
         const size_t smem = (size_t)NW * cells * sizeof(float4);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        launch_chained(kern, dim3((pairs + NW - 1) / NW), dim3(32 * NW), smem, s, a);
+        kern<<<(pairs + NW - 1) / NW, 32 * NW, smem, s>>>(a);
         e = cudaGetLastError();
     };
     if (K <= 4) {
@@ -842,7 +842,7 @@ cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, int K, cudaStr
         const size_t smem = (size_t)NW * cells * sizeof(float4);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return;
-        launch_chained(kern, dim3(b.items), dim3(32 * NW), smem, s, b);
+        kern<<<b.items, 32 * NW, smem, s>>>(b);
         e = cudaGetLastError();
     };
     if (K <= 4) {
