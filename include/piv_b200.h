@@ -199,8 +199,10 @@ int piv_synchronize(piv_engine *e);
 /* Field readback (synchronises).  selection as write_vec_data_general:
  *   0 grid-1 raw candidates, 1 grid-1 filtered, 2 grid-2 raw candidates, 3 grid-2 filtered.
  * For raw selections dx, dy, valid hold Nt_vec*Npeak_save values (candidate-major per
- * vector); for filtered ones Nt_vec.  x, y receive the grid coordinates (Nt_vec).
- * Any output pointer may be NULL. */
+ * vector); for filtered ones Nt_vec.  x, y receive the grid coordinates (Nt_vec), which do
+ * not depend on the pair: in pageable memory they are filled while the GPU works, also when
+ * the call then reports a device error.  dx, dy and valid are written only by a call that
+ * succeeds.  Any output pointer may be NULL. */
 int piv_get_field(piv_engine *e, int selection, float *x, float *y, float *dx, float *dy, uint8_t *valid);
 
 /* Asynchronous readback (no counterpart in the reference, which reads each field back
@@ -208,7 +210,8 @@ int piv_get_field(piv_engine *e, int selection, float *x, float *y, float *dx, f
  * the engine stream, the copy of a selection (0..3, as piv_get_field) into one of two
  * engine-owned pinned slots, together with the device status word of that work, and
  * returns at once with a ticket.  piv_field_wait waits for that copy, reports a device
- * error of its pair (PIV_ERR_DEVICE), and copies the arrays out (any pointer may be NULL).
+ * error of its pair (PIV_ERR_DEVICE), and copies the arrays out (any pointer may be NULL; x
+ * and y as piv_get_field fills them).
  * A caller thus keeps the next pair queued while it reads the previous one:
  *   queue(0); for k: run(k); t[k] = field_async(k); queue(k+1); field_wait(t[k-1]).
  * At most two readbacks are pending (PIV_ERR_STATE otherwise). */

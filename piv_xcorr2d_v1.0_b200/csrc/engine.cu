@@ -11,6 +11,8 @@
 //               fill work list.
 // There are no correlation-plane buffers: the fused kernel keeps them on chip.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cctype>
@@ -742,12 +744,23 @@ void grid_coordinates(const GridGeom &g, float *x, float *y)
     }
 }
 
-// First touch of the caller's pages (fresh ones are mapped on demand), contents unchanged.
-void touch_pages(void *p, size_t bytes)
+// Memory that CUDA knows: pinned, managed or device.
+bool cuda_knows(const void *p)
 {
-    if (!p) return;
-    volatile char *c = static_cast<volatile char *>(p);
-    for (size_t o = 0; o < bytes; o += 4096) c[o] = c[o];
+    cudaPointerAttributes at;
+    return p && cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+}
+
+// Maps the caller's fresh pages (they are mapped on demand, one fault each) while the GPU works.
+// No byte is read or written: another copy may be filling them, and a call that fails leaves them
+// as they were.  Memory that cannot be mapped ahead, or a kernel without the advice, loses nothing.
+void map_pages(void *p, size_t bytes)
+{
+    if (!p || !bytes || cuda_knows(p)) return;
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = (uintptr_t)p & ~(page - 1);
+    madvise(reinterpret_cast<void *>(first), (uintptr_t)p + bytes - first, MADV_POPULATE_WRITE);
+#endif
 }
 
 int validate_params(piv_engine *e, const piv_params &p)
@@ -1260,11 +1273,7 @@ int piv_get_field(piv_engine *e, int sel, float *x, float *y, float *dx, float *
     const bool raw = (sel % 2) == 0;
     const GridState &gs = e->grid[k];
     const size_t Nt = (size_t)gs.gg.Nt_vec, n = raw ? Nt * e->p.Npeak_save : Nt;
-    auto known = [](const void *q) {  // pinned, managed or device memory
-        cudaPointerAttributes at;
-        return q && cudaPointerGetAttributes(&at, q) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
-    };
-    if (known(dx) || known(dy) || known(valid)) {
+    if (cuda_knows(dx) || cuda_knows(dy) || cuda_knows(valid)) {
         // no host access of ours to what CUDA knows: it takes the copies itself
         if ((rc = piv_synchronize(e))) return rc;
         if (dx) CK(cudaMemcpyAsync(dx, raw ? gs.cdx : gs.fx, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
@@ -1275,42 +1284,50 @@ int piv_get_field(piv_engine *e, int sel, float *x, float *y, float *dx, float *
         return PIV_OK;
     }
     // The results pass through two pinned halves: their copies queue behind the work in flight,
-    // and the host's share (grid coordinates, first touch of the caller's pages) runs beside it.
-    struct Part {
+    // and beside it the caller's pages are mapped and the grid coordinates filled in.  dx, dy and
+    // valid are written once the work is known to be without error.
+    struct Array {
         void *dst;
         const void *src;
         size_t bytes;
     };
-    std::vector<Part> parts;
-    auto add = [&](void *dst, const void *src, size_t bytes) {
-        if (!dst) return;
-        for (size_t o = 0; o < bytes; o += e->bounce)
-            parts.push_back({(char *)dst + o, (const char *)src + o, std::min(e->bounce, bytes - o)});
+    const Array arrays[3] = {{dx, raw ? gs.cdx : gs.fx, dx ? n * sizeof(float) : 0},
+                             {dy, raw ? gs.cdy : gs.fy, dy ? n * sizeof(float) : 0},
+                             {valid, raw ? gs.cv : gs.fv, valid ? n : 0}};
+    size_t parts = 0;  // an array's parts are as large as a half
+    for (const Array &a : arrays) parts += (a.bytes + e->bounce - 1) / e->bounce;
+    auto part = [&](size_t i) {
+        const Array *a = arrays;
+        for (size_t np; i >= (np = (a->bytes + e->bounce - 1) / e->bounce); ++a) i -= np;
+        const size_t o = i * e->bounce;
+        return Array{(char *)a->dst + o, (const char *)a->src + o, std::min(e->bounce, a->bytes - o)};
     };
-    add(dx, raw ? gs.cdx : gs.fx, n * sizeof(float));
-    add(dy, raw ? gs.cdy : gs.fy, n * sizeof(float));
-    add(valid, raw ? gs.cv : gs.fv, n);
     CK(cudaMemcpyAsync(e->h_status, e->d_status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     auto queue = [&](size_t i) {
-        CK(cudaMemcpyAsync(e->h_bounce + (i & 1) * e->bounce, parts[i].src, parts[i].bytes, cudaMemcpyDeviceToHost, e->stream));
+        const Array a = part(i);
+        CK(cudaMemcpyAsync(e->h_bounce + (i & 1) * e->bounce, a.src, a.bytes, cudaMemcpyDeviceToHost, e->stream));
         CK(cudaEventRecord(e->ev_bounce[i & 1], e->stream));
         return PIV_OK;
     };
-    for (size_t i = 0; i < parts.size() && i < 2; ++i)
+    for (size_t i = 0; i < parts && i < 2; ++i)
         if ((rc = queue(i))) return rc;
-    for (const Part &p : parts) touch_pages(p.dst, p.bytes);
-    grid_coordinates(gs.gg, x, y);
-    if (parts.empty()) CK(cudaStreamSynchronize(e->stream));
-    for (size_t i = 0; i < parts.size(); ++i) {
+    for (const Array &a : arrays) map_pages(a.dst, a.bytes);
+    const bool coordinates_first = !cuda_knows(x) && !cuda_knows(y);  // no copy in flight can be reading them
+    if (coordinates_first) grid_coordinates(gs.gg, x, y);
+    if (parts == 0) CK(cudaStreamSynchronize(e->stream));
+    for (size_t i = 0; i < parts; ++i) {
         CK(cudaEventSynchronize(e->ev_bounce[i & 1]));
         if (i == 0 && *e->h_status) {
             CK(cudaStreamSynchronize(e->stream));  // the second half's copy is in flight
             break;
         }
-        std::memcpy(parts[i].dst, e->h_bounce + (i & 1) * e->bounce, parts[i].bytes);
-        if (i + 2 < parts.size() && (rc = queue(i + 2))) return rc;
+        const Array a = part(i);
+        std::memcpy(a.dst, e->h_bounce + (i & 1) * e->bounce, a.bytes);
+        if (i + 2 < parts && (rc = queue(i + 2))) return rc;
     }
-    return after_synchronize(e);
+    if ((rc = after_synchronize(e))) return rc;
+    if (!coordinates_first) grid_coordinates(gs.gg, x, y);
+    return PIV_OK;
 }
 
 int piv_field_async(piv_engine *e, int sel, int *ticket)
@@ -1365,11 +1382,12 @@ int piv_field_wait(piv_engine *e, int ticket, float *x, float *y, float *dx, flo
     cudaSetDevice(e->device);
     const GridState &gs = e->grid[r.sel / 2];
     const size_t Nt = (size_t)gs.gg.Nt_vec, n = (r.sel % 2 == 0) ? Nt * e->p.Npeak_save : Nt;
-    // beside the work in flight: grid coordinates, first touch of the caller's pages
-    touch_pages(dx, n * sizeof(float));
-    touch_pages(dy, n * sizeof(float));
-    touch_pages(valid, n);
-    grid_coordinates(gs.gg, x, y);
+    // beside the work in flight, as in piv_get_field
+    map_pages(dx, n * sizeof(float));
+    map_pages(dy, n * sizeof(float));
+    map_pages(valid, n);
+    const bool coordinates_first = !cuda_knows(x) && !cuda_knows(y);
+    if (coordinates_first) grid_coordinates(gs.gg, x, y);
     CK(cudaEventSynchronize(r.ev));
     r.pending = false;
     if (*r.status)
@@ -1379,6 +1397,7 @@ int piv_field_wait(piv_engine *e, int ticket, float *x, float *y, float *dx, flo
     if (dx) std::memcpy(dx, r.dx, n * sizeof(float));
     if (dy) std::memcpy(dy, r.dy, n * sizeof(float));
     if (valid) std::memcpy(valid, r.valid, n);
+    if (!coordinates_first) grid_coordinates(gs.gg, x, y);
     return PIV_OK;
 }
 
