@@ -244,7 +244,10 @@ __device__ __forceinline__ void mhe_apply(const MheGeom &m, const MheFrames &f, 
         // the LUT's entry of byte B of w: the byte takes the place of the base's lowest
         auto entry = [&](uint32_t w, auto bc) {
             uint32_t e;
-            asm volatile("ld.shared.u8 %0, [%1];" : "=r"(e) : "r"(__byte_perm(w, base, 0x7650u | decltype(bc)::value)));
+            asm volatile("ld.shared.u8 %0, [%1];"
+                         : "=r"(e)
+                         : "r"(__byte_perm(w, base, 0x7650u | decltype(bc)::value))
+                         : "memory");
             return e;
         };
         using std::integral_constant;
