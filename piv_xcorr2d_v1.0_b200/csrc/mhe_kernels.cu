@@ -51,11 +51,6 @@ __device__ __forceinline__ bool mhe_words(const uint8_t *p, int pitch, int ws)
     return ((reinterpret_cast<uintptr_t>(p) & 3) == 0) && (pitch % 4 == 0) && (ws % 4 == 0);
 }
 
-// q / d by a multiply with ceil(2^32 / d) and a 32-bit shift: exact while q * d < 2^32
-// (the reciprocal's rounding error then stays below 1/d), which tile sizes here satisfy.
-__device__ __forceinline__ int div_small(int q, uint64_t magic) { return (int)(((uint64_t)q * magic) >> 32); }
-__host__ __device__ inline uint64_t div_magic(int d) { return (0x100000000ull + (uint64_t)d - 1) / (uint64_t)d; }
-
 // One frame, or both of a pair in one launch (blockIdx.y): on small frames, where a launch is a
 // few CTAs, the second frame then costs nothing (enhancement of a pair by two such launches
 // instead of four: 333x251 40 -> 19 us, 1024x1024 21 -> 15).
@@ -75,7 +70,7 @@ struct MheFrames {
 // column, bytes become shared-memory addresses by one or two logic instructions, and the LUT
 // multiplies.  Bounded to 64 registers: 4 CTAs per SM (5 and 6 spill; unbounded 43 -> 49 us).  One
 // frame of 4096x2160: 27.6 -> 21.4 us, of 6600x4400: 52.5 -> 43.  Tiles whose rows are not
-// 4-byte aligned (the odd widths) go byte by byte as before.
+// 4-byte aligned (the odd widths) go byte by byte (ByteLane).
 struct WordLane {
     int c0, r0, n;
     __device__ WordLane(const MheFrames &f, int ws, int lane)
@@ -83,6 +78,37 @@ struct WordLane {
         r0 = (lane * f.lane_magic) >> 16;
         c0 = lane - r0 * f.wpr;
         n = r0 < f.row_step && c0 < f.wpr ? (ws - r0 + f.row_step - 1) / f.row_step : 0;
+    }
+};
+
+// The pixels of a tile one byte at a time, as one lane visits them: every 32nd in row order.  A step
+// is some whole rows and a part of one, which passes the row's end at most once, so nothing is
+// divided after the first pixel.  A warp has one tile, so the latency of its chain of batches is
+// what bounds tiles of 32 px and more, and a division per pixel (two in the second kernel) was twice
+// as long a chain.  One frame of 4095x2159: 25 px tiles 44.3 -> 34.0 us, 40 px 40.2 -> 27.9, 128 px
+// 113.3 -> 60.2, 300 px 592 -> 301.
+template <class T>
+struct ByteLane {
+    T *p;
+    int c, ws, rest;
+    ptrdiff_t step_bytes, wrap;
+    __device__ ByteLane(T *tile, int pitch, int w, int lane) : ws(w)
+    {
+        const int r = lane / w, rows = 32 / w;
+        c = lane - r * w;
+        p = tile + (ptrdiff_t)r * pitch + c;
+        rest = 32 - rows * w;
+        step_bytes = (ptrdiff_t)rows * pitch + rest;
+        wrap = pitch - w;
+    }
+    __device__ void step()
+    {
+        p += step_bytes;
+        c += rest;
+        if (c >= ws) {
+            c -= ws;
+            p += wrap;
+        }
     }
 };
 
@@ -133,17 +159,14 @@ __global__ void __launch_bounds__(256, 4) mhe_hist_kernel(const MheGeom m, const
         }
     } else {
         const int npx = m.ws * m.ws;
-        const uint64_t mg = div_magic(m.ws);
-        for (int base = 0; base < npx; base += 32 * kBatch) {
+        ByteLane<const uint8_t> l(src, in_pitch, m.ws, lane);
+        for (int base = lane; base < npx; base += 32 * kBatch) {
             int v[kBatch];
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
-                const int p = base + k * 32 + lane;
                 v[k] = -1;
-                if (p < npx) {
-                    const int r = div_small(p, mg), c = p - r * m.ws;
-                    v[k] = *(src + (size_t)r * in_pitch + c);
-                }
+                if (base + 32 * k < npx) v[k] = *l.p;
+                l.step();
             }
 #pragma unroll
             for (int k = 0; k < kBatch; ++k)
@@ -277,25 +300,20 @@ __device__ __forceinline__ void mhe_apply(const MheGeom &m, const MheFrames &f, 
         }
     } else {
         const int npx = m.ws * m.ws;
-        const uint64_t mgp = div_magic(m.ws);
-        for (int base = 0; base < npx; base += 32 * kBatch) {
+        ByteLane<const uint8_t> from(src, in_pitch, m.ws, lane);
+        ByteLane<uint8_t> to(dst, out_pitch, m.ws, lane);
+        for (int base = lane; base < npx; base += 32 * kBatch) {
             int px[kBatch];
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
-                const int p = base + k * 32 + lane;
                 px[k] = 0;
-                if (p < npx) {
-                    const int r = div_small(p, mgp), cc = p - r * m.ws;
-                    px[k] = *(src + (size_t)r * in_pitch + cc);
-                }
+                if (base + 32 * k < npx) px[k] = *from.p;
+                from.step();
             }
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
-                const int p = base + k * 32 + lane;
-                if (p < npx) {
-                    const int r = div_small(p, mgp), cc = p - r * m.ws;
-                    dst[(size_t)r * out_pitch + cc] = lut[px[k]];
-                }
+                if (base + 32 * k < npx) *to.p = lut[px[k]];
+                to.step();
             }
         }
     }
