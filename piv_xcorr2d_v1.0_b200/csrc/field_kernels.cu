@@ -655,47 +655,39 @@ __device__ __forceinline__ void merge_exchange_sort(float (&a)[N])
     if constexpr (P > 1) merge_exchange_sort<N, P / 2>(a);
 }
 
-// Median and MAD of one component of a 5x5 neighbourhood that holds an infinity or a NaN
-// (candidates set by the caller).  What fminf and fmaxf make of those depends on the exchanges, so
-// these are median_pass_kernel's, in loops over local memory: rare, and no register is kept for it.
-__device__ __noinline__ float2 median5_nonfinite(const float *src, const uint8_t *flag, int step, int Nx, int Ny,
-                                                 int vx, int vy)
+// Median and MAD of one component of the 5x5 neighbourhood of (vx, vy) by a whole warp, slot q of
+// median_pass_kernel's network in lane q.  For NaN (candidates set by the caller) and medians that
+// are no number: what fminf and fmaxf make of those depends on the exchanges, so these are the
+// network's own.  About 100 instructions a neighbourhood; every lane gets the result.  Not inlined:
+// inlined, the 511 x 269 grid without NaN took 53 us instead of 51.
+__device__ __noinline__ float2 median5_warp(const float *src, const uint8_t *flag, int step, int Nx, int Ny, int vx,
+                                               int vy, int lane)
 {
+    const unsigned all = 0xffffffffu;
     const float inf = __int_as_float(0x7f800000);
-    float w[32];
-    int n = 0;
-#pragma unroll 1
-    for (int q = 0; q < 32; ++q) {
-        const int x = vx + q % 5 - 2, y = vy + q / 5 - 2;
-        w[q] = inf;
-        if (q < 25 && q != 12 && x >= 0 && x < Nx && y >= 0 && y < Ny && flag[(size_t)(y * Nx + x) * step]) {
-            w[q] = src[(size_t)(y * Nx + x) * step];
-            ++n;
+    const int x = vx + lane % 5 - 2, y = vy + lane / 5 - 2;
+    bool ok = lane < 25 && lane != 12 && x >= 0 && x < Nx && y >= 0 && y < Ny;
+    const size_t id = (size_t)(ok ? y * Nx + x : 0) * step;
+    ok = ok && flag[id];
+    float w = ok ? src[id] : inf;
+    const int n = __popc(__ballot_sync(all, ok));
+    auto merge = [&](int k) {  // the exchanges of size k
+#pragma unroll
+        for (int j = k / 2; j > 0; j /= 2) {
+            const float o = __shfl_xor_sync(all, w, j);
+            w = ((lane & k) != 0) != ((lane & j) != 0) ? fmaxf(w, o) : fminf(w, o);
         }
-    }
-    float med = 0.f, mad = 0.f;
-#pragma unroll 1
-    for (int round = 0; round < 2; ++round) {
-        // the whole network, then its final merge stage
-#pragma unroll 1
-        for (int k = round ? 32 : 2; k <= 32; k *= 2)
-#pragma unroll 1
-            for (int j = k / 2; j > 0; j /= 2)
-#pragma unroll 1
-                for (int i = 0; i < 32; ++i) {
-                    const int l = i ^ j;
-                    if (l < i) continue;
-                    const float lo = fminf(w[i], w[l]), hi = fmaxf(w[i], w[l]);
-                    w[i] = (i & k) ? hi : lo;
-                    w[l] = (i & k) ? lo : hi;
-                }
-        mad = n % 2 ? w[n / 2] : (w[n / 2] + w[n / 2 - 1]) / 2;
-        if (round) break;
-        med = mad;
-#pragma unroll 1
-        for (int q = 0; q < 32; ++q) w[q] = q < n ? fabsf(w[q] - med) : inf;
-    }
-    return make_float2(med, mad);
+    };
+    auto median = [&]() {
+        const float hi = __shfl_sync(all, w, n / 2), lo = __shfl_sync(all, w, (n / 2 - 1) & 31);
+        return n % 2 ? hi : (hi + lo) / 2;
+    };
+#pragma unroll
+    for (int k = 2; k <= 32; k *= 2) merge(k);
+    const float med = median();
+    w = lane < n ? fabsf(w - med) : inf;
+    merge(32);
+    return make_float2(med, median());
 }
 
 // The 5x5 stencil (the usual one): two threads per vector, one for each component, which meet by
@@ -706,7 +698,11 @@ __device__ __noinline__ float2 median5_nonfinite(const float *src, const uint8_t
 // min(lower[i], upper[11 - i]).  What bounds it: the latency of the straight-line code on small
 // grids, issue slots on large ones.  Validation of a grid (two median passes, fill, smoothing), one
 // thread per vector with the general network -> this: 21 x 16 vectors 34 -> 23 us, 411 x 274
-// 64 -> 43 us, 384 x 509 98 -> 63 us.  Other stencils keep median_pass_kernel: the exchanges and
+// 64 -> 43 us, 384 x 509 98 -> 63 us.  Neighbourhoods that need the network's own exchanges
+// (median5_warp) are taken by the whole warp one after another: with 5 % of the candidates NaN
+// 511 x 269 vectors take 117 us (51 without; one thread per vector and the general network 91, a
+// thread's own loops over local memory 202), with infinities alone 57 to 75.  Other stencils keep
+// median_pass_kernel: the exchanges and
 // the two halves of the MAD are laid out for exactly 24 neighbours.
 __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
 {
@@ -722,7 +718,7 @@ __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
     const float inf = __int_as_float(0x7f800000);
     float s[24];
     int n = 0;
-    bool odd = false;
+    bool odd = false;  // a NaN
 #pragma unroll
     for (int q = 0; q < 25; ++q) {
         if (q == 12) continue;  // the centre
@@ -733,15 +729,11 @@ __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
         const float f = src[id];
         s[q < 12 ? q : q - 1] = ok ? f : inf;
         n += ok;
-        odd |= ok && !(fabsf(f) < inf);
+        odd |= ok && f != f;
     }
     merge_exchange_sort<24, 16>(s);
     float med, mad;
-    if (odd) {
-        const float2 m = median5_nonfinite(src, flag, step, a.Nx, a.Ny, vx, vy);
-        med = m.x;
-        mad = m.y;
-    } else if (n == 24) {
+    if (n == 24) {
         med = (s[12] + s[11]) / 2;
         float lo = 0.f, hi = inf;
 #pragma unroll
@@ -763,10 +755,21 @@ __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
         bitonic_step<32, 32, 16>(w);
         mad = median_sorted<32>(w, n);
     }
+    const bool judged = n >= a.minN && n >= 1;
+    for (unsigned todo = __ballot_sync(0xffffffffu, judged && (odd || !(fabsf(med) < inf))); todo; todo &= todo - 1) {
+        const int q = __ffs(todo) - 1;  // component q & 1, as this lane's by its own parity
+        const int qx = __shfl_sync(0xffffffffu, vx, q), qy = __shfl_sync(0xffffffffu, vy, q);
+        const float *from = a.ix ? (q & 1 ? a.iy : a.ix) : (q & 1 ? a.cdy : a.cdx);
+        const float2 m = median5_warp(from, flag, step, a.Nx, a.Ny, qx, qy, threadIdx.x & 31);
+        if ((threadIdx.x & 31) == q) {
+            med = m.x;
+            mad = m.y;
+        }
+    }
     // median_filtering's decision (median_decide): the first valid candidate with both residuals
     // below the threshold
     const float epsilon = 0.1f;
-    bool found = !(n >= a.minN && n >= 1), ok = false;
+    bool found = !judged, ok = false;
     float r = 0.f;
     for (int i = 0; i < a.Nps; ++i) {
         const size_t c = (size_t)v * a.Nps + i;
