@@ -41,9 +41,14 @@ __device__ __forceinline__ float ext_field(const float *f, int Nx, int Ny, int m
 constexpr int kDeformRows = 32, kDeformThreads = 128, kDeformMinCtas = 600;
 constexpr int kDeformFar = 1 << 21;  // positions that the addition of 1.5 * 2^23 splits, with room to spare
 
-// One pixel at (px, py): taps may lie outside the frame, and the position may be any number.
+// One pixel at (px, py): taps may lie outside the frame, and the position may be any number or none.
+// Without the first line a predictor with NaN in 1 % of its vectors took 28.6 us at 2048x1536 and
+// spacing 16 (15.0 with it, 14.7 without NaN): eight such calls in a row for a run of pixels.
 __device__ __noinline__ float deform_any(const Frame8 &f, float px, float py, int col_off, int row_off)
 {
+    const float inf = __int_as_float(0x7f800000);
+    // no number: an infinite position's taps lie outside, and its weights times their zeros are NaN
+    if (!(fabsf(px) < inf && fabsf(py) < inf)) return __int_as_float(0x7fffffff);
     const int i_x = (int)floorf(px), i_y = (int)floorf(py);
     const float a_x = __fsub_rn(px, (float)i_x), a_y = __fsub_rn(py, (float)i_y);
     float p[4];
