@@ -635,12 +635,19 @@ __device__ __forceinline__ void peak_window_merge(const XcorrArgs &a, const floa
 // Residency asked of the register allocation (the second __launch_bounds__ argument), where
 // the compiler's own choice leaves the SM's shared memory unused: 64x64 with 2 windows per CTA
 // of 128 threads (68 KB: 3 CTAs at 168 registers and 160 bytes of spills, 0.547 ms a grid-1
-// launch at 6600x4400; unbounded 217 registers and 2 CTAs, 0.685), 32x32 with 4 windows per CTA
-// of 128 threads (5 CTAs at 96 registers).
+// launch at 6600x4400; unbounded 217 registers and 2 CTAs, 0.685), 32x64 with 4 windows per 128
+// threads or 2 per 64 (12 warps at 168 registers and 224 to 256 bytes of spills; a launch at
+// 4096x2160 and spacing 8x16 668 and 692 us, unbounded at 213 registers 726 and 712, 1024x768
+// and spacing 16x32 19.3 and 20.8 us against 24.1 and 23.7), 32x32 with 4 windows per CTA of 128
+// threads (5 CTAs at 96 registers).
 template <int WSX, int WSY, int B, int NT>
 constexpr int xcorr_min_ctas()
 {
-    return (WSX == 32 && WSY == 32 && B == 4 && NT == 128) ? 5 : (WSX == 64 && WSY == 64 && B == 2 && NT == 128) ? 3 : 1;
+    if (WSX == 32 && WSY == 32 && B == 4 && NT == 128) return 5;
+    if (WSX == 64 && WSY == 64 && B == 2 && NT == 128) return 3;
+    if (WSX == 32 && WSY == 64 && B == 4 && NT == 128) return 3;
+    if (WSX == 32 && WSY == 64 && B == 2 && NT == 64) return 6;
+    return 1;
 }
 
 template <int WSX, int WSY, int B, int NT, int K, bool DEF>
