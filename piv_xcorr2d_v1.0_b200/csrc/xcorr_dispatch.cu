@@ -1,5 +1,5 @@
 // xcorr_dispatch.cu -- window shape and variant -> instantiated fused correlation kernel.
-// Every shape (WSX, WSY) is compiled in its own translation unit (xcorr_shape_*.cu) in
+// Every shape (WSX, WSY) is compiled in translation units of its own (xcorr_shape_*.cu) in
 // several variants (B windows per CTA, NT threads per CTA); the first listed variant of a
 // shape is its default, the engine's autotuner may pick another one per grid.
 #include <cstring>
@@ -9,8 +9,9 @@
 
 namespace piv {
 
-template <int WSX, int WSY, int B, int NT>
-cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t s);
+// K: the most saved peaks, 4 or 8
+template <int WSX, int WSY, int B, int NT, int K>
+cudaError_t launch_shape(const XcorrArgs &a, bool deformed, cudaStream_t s);
 
 #define PIV_XCORR_VARIANTS(X) \
     X(8, 8, 32, 128) \
@@ -60,24 +61,28 @@ cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t 
     X(32, 64, 2, 64) \
     X(32, 64, 2, 128)
 
-#define PIV_X(WX, WY, B, NT) extern template cudaError_t launch_shape<WX, WY, B, NT>(const XcorrArgs &, bool, int, cudaStream_t);
+#define PIV_X(WX, WY, B, NT) \
+    extern template cudaError_t launch_shape<WX, WY, B, NT, 4>(const XcorrArgs &, bool, cudaStream_t); \
+    extern template cudaError_t launch_shape<WX, WY, B, NT, 8>(const XcorrArgs &, bool, cudaStream_t);
 PIV_XCORR_VARIANTS(PIV_X)
 #undef PIV_X
 // the 2x2-block form (four windows of two window rows per CTA), listed after the shape's
 // row-major variants
-template <int WSX, int WSY, int NT>
-cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, int K, cudaStream_t s);
-extern template cudaError_t launch_shape_block<32, 32, 128>(const XcorrArgs &, bool, int, cudaStream_t);
+template <int WSX, int WSY, int NT, int K>
+cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, cudaStream_t s);
+extern template cudaError_t launch_shape_block<32, 32, 128, 4>(const XcorrArgs &, bool, cudaStream_t);
+extern template cudaError_t launch_shape_block<32, 32, 128, 8>(const XcorrArgs &, bool, cudaStream_t);
 
 // the warp form (a window pair per warp, four warps per CTA), listed before them
-template <int NW>
-cudaError_t launch_pair(const XcorrArgs &a, bool deformed, int K, cudaStream_t s);
-extern template cudaError_t launch_pair<4>(const XcorrArgs &, bool, int, cudaStream_t);
+template <int NW, int K>
+cudaError_t launch_pair(const XcorrArgs &a, bool deformed, cudaStream_t s);
+extern template cudaError_t launch_pair<4, 4>(const XcorrArgs &, bool, cudaStream_t);
+extern template cudaError_t launch_pair<4, 8>(const XcorrArgs &, bool, cudaStream_t);
 
 // Variants of the persistent batch launch (two per shape; the batch autotuner picks one
 // per shape group).
-template <int WSX, int WSY, int B, int NT>
-cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaStream_t s);
+template <int WSX, int WSY, int B, int NT, int K>
+cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, cudaStream_t s);
 #define PIV_XCORR_BATCH_VARIANTS(X) \
     X(8, 8, 32, 128) \
     X(8, 8, 16, 128) \
@@ -104,21 +109,23 @@ cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaSt
     X(64, 32, 2, 64) \
     X(32, 64, 4, 128) \
     X(32, 64, 2, 64)
-#define PIV_X(WX, WY, B, NT) extern template cudaError_t launch_shape_batch<WX, WY, B, NT>(const XcorrBatch &, bool, int, cudaStream_t);
+#define PIV_X(WX, WY, B, NT) \
+    extern template cudaError_t launch_shape_batch<WX, WY, B, NT, 4>(const XcorrBatch &, bool, cudaStream_t); \
+    extern template cudaError_t launch_shape_batch<WX, WY, B, NT, 8>(const XcorrBatch &, bool, cudaStream_t);
 PIV_XCORR_BATCH_VARIANTS(PIV_X)
 #undef PIV_X
 
 namespace {
 struct Variant {
     int wsx, wsy, B, NT;
-    cudaError_t (*fn)(const XcorrArgs &, bool, int, cudaStream_t);
+    cudaError_t (*fn[2])(const XcorrArgs &, bool, cudaStream_t);  // up to 4 saved peaks, up to 8
 };
 const Variant kVariants[] = {
-    {32, 32, 8, 128, &launch_pair<4>},
-#define PIV_X(WX, WY, B, NT) {WX, WY, B, NT, &launch_shape<WX, WY, B, NT>},
+    {32, 32, 8, 128, {&launch_pair<4, 4>, &launch_pair<4, 8>}},
+#define PIV_X(WX, WY, B, NT) {WX, WY, B, NT, {&launch_shape<WX, WY, B, NT, 4>, &launch_shape<WX, WY, B, NT, 8>}},
     PIV_XCORR_VARIANTS(PIV_X)
 #undef PIV_X
-    {32, 32, 4, 128, &launch_shape_block<32, 32, 128>},
+    {32, 32, 4, 128, {&launch_shape_block<32, 32, 128, 4>, &launch_shape_block<32, 32, 128, 8>}},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
@@ -152,18 +159,20 @@ bool xcorr_variant_shape(int wsx, int wsy, int variant, int *B, int *NT)
     return true;
 }
 
-template <int NW>
-cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, int K, cudaStream_t s);
-extern template cudaError_t launch_pair_batch<4>(const XcorrBatch &, bool, int, cudaStream_t);
+template <int NW, int K>
+cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, cudaStream_t s);
+extern template cudaError_t launch_pair_batch<4, 4>(const XcorrBatch &, bool, cudaStream_t);
+extern template cudaError_t launch_pair_batch<4, 8>(const XcorrBatch &, bool, cudaStream_t);
 
 namespace {
 struct BatchVariant {
     int wsx, wsy, B, NT;
-    cudaError_t (*fn)(const XcorrBatch &, bool, int, cudaStream_t);
+    cudaError_t (*fn[2])(const XcorrBatch &, bool, cudaStream_t);
 };
 const BatchVariant kBatchVariants[] = {
-    {32, 32, 8, 128, &launch_pair_batch<4>},
-#define PIV_X(WX, WY, B, NT) {WX, WY, B, NT, &launch_shape_batch<WX, WY, B, NT>},
+    {32, 32, 8, 128, {&launch_pair_batch<4, 4>, &launch_pair_batch<4, 8>}},
+#define PIV_X(WX, WY, B, NT) \
+    {WX, WY, B, NT, {&launch_shape_batch<WX, WY, B, NT, 4>, &launch_shape_batch<WX, WY, B, NT, 8>}},
     PIV_XCORR_BATCH_VARIANTS(PIV_X)
 #undef PIV_X
 };
@@ -201,7 +210,7 @@ cudaError_t launch_xcorr_batch(int wsx, int wsy, int variant, const XcorrBatch &
         if (why) *why = "window shape has no batch launch";
         return cudaErrorInvalidValue;
     }
-    return v->fn(b, deformed, K, s);
+    return v->fn[K > 4](b, deformed, s);
 }
 
 cudaError_t launch_xcorr(const XcorrArgs &a, bool deformed, cudaStream_t s, const char **why, int variant)
@@ -216,7 +225,7 @@ cudaError_t launch_xcorr(const XcorrArgs &a, bool deformed, cudaStream_t s, cons
         if (why) *why = "window shape not built into this engine";
         return cudaErrorInvalidValue;
     }
-    return v->fn(a, deformed, a.g.Nps <= 4 ? 4 : 8, s);
+    return v->fn[a.g.Nps > 4](a, deformed, s);
 }
 
 }  // namespace piv

@@ -737,10 +737,11 @@ __global__ void __launch_bounds__(NT, (xcorr_min_ctas<WSX, WSY, B, NT>())) xcorr
 }
 
 // ------------------------------------------------------------------------------
-// Launch of one instantiated shape (explicitly instantiated in xcorr_shape_*.cu).
+// Launch of one instantiated shape, K saved peaks at most (explicitly instantiated in
+// xcorr_shape_*.cu).
 // ------------------------------------------------------------------------------
-template <int WSX, int WSY, int B, int NT>
-cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t s)
+template <int WSX, int WSY, int B, int NT, int K>
+cudaError_t launch_shape(const XcorrArgs &a, bool deformed, cudaStream_t s)
 {
     if (a.w_end <= a.w_first) return cudaSuccess;
     const int n = a.w_end - (a.w_first & ~1);  // CTAs start at an even window (pairing)
@@ -753,25 +754,20 @@ cudaError_t launch_shape(const XcorrArgs &a, bool deformed, int K, cudaStream_t 
         kern<<<grid, NT, smem, s>>>(a);
         e = cudaGetLastError();
     };
-    if (K <= 4) {
-        if (deformed) go(xcorr_peak_kernel<WSX, WSY, B, NT, 4, true>);
-        else go(xcorr_peak_kernel<WSX, WSY, B, NT, 4, false>);
-    } else {
-        if (deformed) go(xcorr_peak_kernel<WSX, WSY, B, NT, 8, true>);
-        else go(xcorr_peak_kernel<WSX, WSY, B, NT, 8, false>);
-    }
+    if (deformed) go(xcorr_peak_kernel<WSX, WSY, B, NT, K, true>);
+    else go(xcorr_peak_kernel<WSX, WSY, B, NT, K, false>);
     return e;
 }
 
 // Launch of the 2x2-block form (four windows per CTA): the blocks of the launch's window rows
 // (rounded out to whole block rows; windows outside [w_first, w_end) are computed, not
 // written).  An odd row of windows has no whole pairs of columns: the row-major form then.
-template <int WSX, int WSY, int NT>
-cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, int K, cudaStream_t s)
+template <int WSX, int WSY, int NT, int K>
+cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, cudaStream_t s)
 {
     if (a.w_end <= a.w_first) return cudaSuccess;
     const int nx = a.g.Nx_vec;
-    if (nx % 2) return launch_shape<WSX, WSY, 4, NT>(a, deformed, K, s);
+    if (nx % 2) return launch_shape<WSX, WSY, 4, NT, K>(a, deformed, s);
     const int by0 = (a.w_first / nx) >> 1, by1 = ((a.w_end - 1) / nx) >> 1;
     const size_t smem = (size_t)2 * Plane<WSX, WSY>::PW * sizeof(float4);
     dim3 grid((unsigned)((nx >> 1) * (by1 - by0 + 1)));
@@ -782,20 +778,15 @@ cudaError_t launch_shape_block(const XcorrArgs &a, bool deformed, int K, cudaStr
         kern<<<grid, NT, smem, s>>>(a);
         e = cudaGetLastError();
     };
-    if (K <= 4) {
-        if (deformed) go(xcorr_block_kernel<WSX, WSY, NT, 4, true>);
-        else go(xcorr_block_kernel<WSX, WSY, NT, 4, false>);
-    } else {
-        if (deformed) go(xcorr_block_kernel<WSX, WSY, NT, 8, true>);
-        else go(xcorr_block_kernel<WSX, WSY, NT, 8, false>);
-    }
+    if (deformed) go(xcorr_block_kernel<WSX, WSY, NT, K, true>);
+    else go(xcorr_block_kernel<WSX, WSY, NT, K, false>);
     return e;
 }
 
 // Launch of a batch: items = sum over pairs of ceil(windows / B), first[] their prefix
 // sums; one CTA per item.
-template <int WSX, int WSY, int B, int NT>
-cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaStream_t s)
+template <int WSX, int WSY, int B, int NT, int K>
+cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, cudaStream_t s)
 {
     if (b.items <= 0) return cudaSuccess;
     const size_t smem = (size_t)(B / 2) * Plane<WSX, WSY>::PW * sizeof(float4);
@@ -806,19 +797,14 @@ cudaError_t launch_shape_batch(const XcorrBatch &b, bool deformed, int K, cudaSt
         kern<<<b.items, NT, smem, s>>>(b);
         e = cudaGetLastError();
     };
-    if (K <= 4) {
-        if (deformed) go(xcorr_batch_kernel<WSX, WSY, B, NT, 4, true>);
-        else go(xcorr_batch_kernel<WSX, WSY, B, NT, 4, false>);
-    } else {
-        if (deformed) go(xcorr_batch_kernel<WSX, WSY, B, NT, 8, true>);
-        else go(xcorr_batch_kernel<WSX, WSY, B, NT, 8, false>);
-    }
+    if (deformed) go(xcorr_batch_kernel<WSX, WSY, B, NT, K, true>);
+    else go(xcorr_batch_kernel<WSX, WSY, B, NT, K, false>);
     return e;
 }
 
 // Launches of the warp form (two windows per warp, NW warps per CTA).
-template <int NW>
-cudaError_t launch_pair(const XcorrArgs &a, bool deformed, int K, cudaStream_t s)
+template <int NW, int K>
+cudaError_t launch_pair(const XcorrArgs &a, bool deformed, cudaStream_t s)
 {
     if (a.w_end <= a.w_first) return cudaSuccess;
     const int pairs = (a.w_end - (a.w_first & ~1) + 1) / 2;  // warps start at an even window
@@ -830,18 +816,13 @@ cudaError_t launch_pair(const XcorrArgs &a, bool deformed, int K, cudaStream_t s
         kern<<<(pairs + NW - 1) / NW, 32 * NW, smem, s>>>(a);
         e = cudaGetLastError();
     };
-    if (K <= 4) {
-        if (deformed) go(xcorr_pair_kernel<NW, 4, true>, PairShared<4>::CELLS);
-        else go(xcorr_pair_kernel<NW, 4, false>, PairShared<4>::CELLS);
-    } else {
-        if (deformed) go(xcorr_pair_kernel<NW, 8, true>, PairShared<8>::CELLS);
-        else go(xcorr_pair_kernel<NW, 8, false>, PairShared<8>::CELLS);
-    }
+    if (deformed) go(xcorr_pair_kernel<NW, K, true>, PairShared<K>::CELLS);
+    else go(xcorr_pair_kernel<NW, K, false>, PairShared<K>::CELLS);
     return e;
 }
 
-template <int NW>
-cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, int K, cudaStream_t s)
+template <int NW, int K>
+cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, cudaStream_t s)
 {
     if (b.items <= 0) return cudaSuccess;
     cudaError_t e = cudaSuccess;
@@ -852,14 +833,25 @@ cudaError_t launch_pair_batch(const XcorrBatch &b, bool deformed, int K, cudaStr
         kern<<<b.items, 32 * NW, smem, s>>>(b);
         e = cudaGetLastError();
     };
-    if (K <= 4) {
-        if (deformed) go(xcorr_pair_batch_kernel<NW, 4, true>, PairShared<4>::CELLS);
-        else go(xcorr_pair_batch_kernel<NW, 4, false>, PairShared<4>::CELLS);
-    } else {
-        if (deformed) go(xcorr_pair_batch_kernel<NW, 8, true>, PairShared<8>::CELLS);
-        else go(xcorr_pair_batch_kernel<NW, 8, false>, PairShared<8>::CELLS);
-    }
+    if (deformed) go(xcorr_pair_batch_kernel<NW, K, true>, PairShared<K>::CELLS);
+    else go(xcorr_pair_batch_kernel<NW, K, false>, PairShared<K>::CELLS);
     return e;
 }
+
+// A shape's kernels are compiled in parts (PIV_K 4 or 8 saved peaks, PIV_BATCH 0 or 1), because the
+// driver loads a whole module with the first of its kernels and a program rarely needs two parts.
+// The first use in a process of 64x64 took 25.5 ms in one module, 9.5 in parts; 32x32 15.5 -> 7.1,
+// 48x48 18.4 -> 7.2.
+#ifdef PIV_K
+#if PIV_BATCH
+#define PIV_SHAPE(WX, WY, B, NT)
+#define PIV_SHAPE_BATCH(WX, WY, B, NT) \
+    template cudaError_t launch_shape_batch<WX, WY, B, NT, PIV_K>(const XcorrBatch &, bool, cudaStream_t);
+#else
+#define PIV_SHAPE(WX, WY, B, NT) \
+    template cudaError_t launch_shape<WX, WY, B, NT, PIV_K>(const XcorrArgs &, bool, cudaStream_t);
+#define PIV_SHAPE_BATCH(WX, WY, B, NT)
+#endif
+#endif
 
 }  // namespace piv

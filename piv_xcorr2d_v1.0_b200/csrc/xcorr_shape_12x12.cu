@@ -3,9 +3,9 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<12, 12, 16, 96>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<12, 12, 8, 96>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<12, 12, 16, 192>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<12, 12, 16, 96>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<12, 12, 8, 96>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(12, 12, 16, 96)
+PIV_SHAPE(12, 12, 8, 96)
+PIV_SHAPE(12, 12, 16, 192)
+PIV_SHAPE_BATCH(12, 12, 16, 96)
+PIV_SHAPE_BATCH(12, 12, 8, 96)
 }

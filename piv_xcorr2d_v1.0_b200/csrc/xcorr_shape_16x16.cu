@@ -3,10 +3,10 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<16, 16, 16, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<16, 16, 8, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<16, 16, 16, 256>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<16, 16, 4, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<16, 16, 16, 128>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<16, 16, 8, 128>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(16, 16, 16, 128)
+PIV_SHAPE(16, 16, 8, 128)
+PIV_SHAPE(16, 16, 16, 256)
+PIV_SHAPE(16, 16, 4, 64)
+PIV_SHAPE_BATCH(16, 16, 16, 128)
+PIV_SHAPE_BATCH(16, 16, 8, 128)
 }

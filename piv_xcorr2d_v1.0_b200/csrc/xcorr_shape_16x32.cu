@@ -3,9 +3,9 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<16, 32, 8, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<16, 32, 4, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<16, 32, 8, 256>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<16, 32, 8, 128>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<16, 32, 4, 64>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(16, 32, 8, 128)
+PIV_SHAPE(16, 32, 4, 64)
+PIV_SHAPE(16, 32, 8, 256)
+PIV_SHAPE_BATCH(16, 32, 8, 128)
+PIV_SHAPE_BATCH(16, 32, 4, 64)
 }

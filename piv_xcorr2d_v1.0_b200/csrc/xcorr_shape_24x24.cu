@@ -3,10 +3,10 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<24, 24, 8, 96>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 24, 4, 96>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 24, 8, 192>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 24, 2, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<24, 24, 8, 96>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<24, 24, 4, 96>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(24, 24, 8, 96)
+PIV_SHAPE(24, 24, 4, 96)
+PIV_SHAPE(24, 24, 8, 192)
+PIV_SHAPE(24, 24, 2, 64)
+PIV_SHAPE_BATCH(24, 24, 8, 96)
+PIV_SHAPE_BATCH(24, 24, 4, 96)
 }

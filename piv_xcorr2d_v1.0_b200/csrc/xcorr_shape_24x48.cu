@@ -3,10 +3,10 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<24, 48, 4, 96>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 48, 2, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 48, 4, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<24, 48, 8, 192>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<24, 48, 4, 96>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<24, 48, 2, 64>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(24, 48, 4, 96)
+PIV_SHAPE(24, 48, 2, 64)
+PIV_SHAPE(24, 48, 4, 128)
+PIV_SHAPE(24, 48, 8, 192)
+PIV_SHAPE_BATCH(24, 48, 4, 96)
+PIV_SHAPE_BATCH(24, 48, 2, 64)
 }

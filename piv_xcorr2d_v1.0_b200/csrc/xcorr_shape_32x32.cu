@@ -3,12 +3,15 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_pair<4>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<32, 32, 4, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<32, 32, 2, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<32, 32, 8, 256>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<32, 32, 4, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_block<32, 32, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<32, 32, 4, 128>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_pair_batch<4>(const XcorrBatch &, bool, int, cudaStream_t);
+#if PIV_BATCH
+template cudaError_t launch_pair_batch<4, PIV_K>(const XcorrBatch &, bool, cudaStream_t);
+#else
+template cudaError_t launch_pair<4, PIV_K>(const XcorrArgs &, bool, cudaStream_t);
+template cudaError_t launch_shape_block<32, 32, 128, PIV_K>(const XcorrArgs &, bool, cudaStream_t);
+#endif
+PIV_SHAPE(32, 32, 4, 128)
+PIV_SHAPE(32, 32, 2, 64)
+PIV_SHAPE(32, 32, 8, 256)
+PIV_SHAPE(32, 32, 4, 64)
+PIV_SHAPE_BATCH(32, 32, 4, 128)
 }

@@ -3,9 +3,9 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<64, 32, 4, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<64, 32, 2, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<64, 32, 2, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<64, 32, 4, 128>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<64, 32, 2, 64>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(64, 32, 4, 128)
+PIV_SHAPE(64, 32, 2, 64)
+PIV_SHAPE(64, 32, 2, 128)
+PIV_SHAPE_BATCH(64, 32, 4, 128)
+PIV_SHAPE_BATCH(64, 32, 2, 64)
 }

@@ -3,10 +3,10 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<64, 64, 2, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<64, 64, 4, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<64, 64, 2, 64>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<64, 64, 4, 256>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<64, 64, 2, 128>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<64, 64, 4, 128>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(64, 64, 2, 128)
+PIV_SHAPE(64, 64, 4, 128)
+PIV_SHAPE(64, 64, 2, 64)
+PIV_SHAPE(64, 64, 4, 256)
+PIV_SHAPE_BATCH(64, 64, 2, 128)
+PIV_SHAPE_BATCH(64, 64, 4, 128)
 }

@@ -3,9 +3,9 @@
 #include "xcorr_kernel.cuh"
 
 namespace piv {
-template cudaError_t launch_shape<8, 8, 32, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<8, 8, 16, 128>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape<8, 8, 32, 256>(const XcorrArgs &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<8, 8, 32, 128>(const XcorrBatch &, bool, int, cudaStream_t);
-template cudaError_t launch_shape_batch<8, 8, 16, 128>(const XcorrBatch &, bool, int, cudaStream_t);
+PIV_SHAPE(8, 8, 32, 128)
+PIV_SHAPE(8, 8, 16, 128)
+PIV_SHAPE(8, 8, 32, 256)
+PIV_SHAPE_BATCH(8, 8, 32, 128)
+PIV_SHAPE_BATCH(8, 8, 16, 128)
 }
