@@ -46,6 +46,7 @@ struct GenericPlan {
     int fx[12], fy[12];
     uint32_t mx[12], my[12], px[12], py[12], dx;
     int in_smem;  // 1: the plane in shared memory, 0: in the CTA's workspace slab
+    int rows;     // rows that a warp covers in one step
     int any;      // a radix above 7 (prime up to 251): the local-array stage
 };
 
@@ -299,12 +300,23 @@ __device__ __forceinline__ void gblock_best(float &v, int &i, int &cnt, float *r
     }
 }
 
+// How a warp covers rows of nx points: one row at a time, or 32 / nx rows where they are narrower
+// than the warp (one row at a time left 28 of 32 lanes idle at 4 x 1024: a launch at 2048x1536 503
+// us, 212 this way).  A lane's row of those and its first column are a table in shared memory, 2
+// bytes each: kept in registers over the windows they spilled others, and 12 bytes each cost some
+// windows a resident CTA.
+__device__ __forceinline__ uint16_t row_lane(int nx, int rows, int lane)
+{
+    const int row = rows > 1 ? lane / nx : 0, col = lane - row * nx;
+    return (uint16_t)(row < rows ? row << 10 | col : 1023);  // past every column: an idle lane
+}
+
 // The search region's local maxima, top-K list per thread (rows by warp, columns by lane, so a
 // thread meets them in ascending index order), then per warp, then over the warps: pv, pi get
 // the Nps best.  Returns the count (thread 0).
 template <int K, class Plane>
-__device__ __forceinline__ int gpeaks(const Plane &P, int Nps, int nx, int ilo, int ihi, int jlo, int jhi, float *pv,
-                                      int *pi, PeakPart *parts)
+__device__ __forceinline__ int gpeaks(const Plane &P, int rows, const uint16_t *lanes, int Nps, int nx, int ilo, int ihi, int jlo,
+                                      int jhi, float *pv, int *pi, PeakPart *parts)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float tiny = __int_as_float(1);  // v >= max(neighbours, tiny)  <=>  v > 0 and a local maximum
@@ -316,8 +328,9 @@ __device__ __forceinline__ int gpeaks(const Plane &P, int Nps, int nx, int ilo, 
         ti[k] = INT_MAX;
     }
     int cnt = 0;
-    for (int j = jlo + warp; j <= jhi; j += kGenWarps)
-        for (int i = ilo + lane; i <= ihi; i += 32) {
+    const int at = lanes[lane];
+    for (int j = jlo + warp * rows + (at >> 10); j <= jhi; j += kGenWarps * rows)
+        for (int i = ilo + (at & 1023); i <= ihi; i += 32) {
             const float v = P(i, j);
             const float m = fmaxf(fmaxf(P(i - 1, j), P(i + 1, j)), fmaxf(fmaxf(P(i, j - 1), P(i, j + 1)), tiny));
             if (v >= m) {
@@ -378,6 +391,7 @@ __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel
     const int nx = g.ws_x, ny = g.ws_y, N = nx * ny, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ PeakPart parts[kGenWarps];
+    __shared__ uint16_t s_lanes[32];
     float2 *Wx = reinterpret_cast<float2 *>(gsm);
     float2 *Wy = Wx + nx;
     int *Sx = reinterpret_cast<int *>(Wy + ny);  // shifted column -> storage column
@@ -395,6 +409,7 @@ __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel
     else
         plane = gplane + (size_t)blockIdx.x * N;
 
+    if (tid < 32) s_lanes[tid] = row_lane(nx, pl.rows, tid);
     // tables: forward twiddles (FP64, rounded once) and the index maps
     for (int t = tid; t < nx; t += kGenThreads) {
         double s, c;
@@ -425,10 +440,11 @@ __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel
             const size_t px = (size_t)(iy * g.sp_y - g.Ny_left + a.f1.my) * a.f1.pitch + ix * g.sp_x - g.Nx_left + a.f1.mx;
             const uint8_t *p1 = a.f1.base + px, *p2 = a.f2.base + px;
             const float *pd = DEF ? a.def + (size_t)(iy * g.sp_y) * a.def_pitch + ix * g.sp_x : nullptr;
-            for (int r = warp; r < ny; r += kGenWarps) {
+            const int at = s_lanes[lane];
+            for (int r = warp * pl.rows + (at >> 10); r < ny; r += kGenWarps * pl.rows) {
                 float2 *row = plane + Py[r];
 #pragma unroll 4
-                for (int i = lane; i < nx; i += 32) {
+                for (int i = at & 1023; i < nx; i += 32) {
                     const float v1 = (float)p1[(size_t)r * a.f1.pitch + i];
                     float v2;
                     if constexpr (DEF) v2 = pd[(size_t)r * a.def_pitch + i];
@@ -447,9 +463,10 @@ __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel
         const float2 dc = plane[0];
         const bool dead = dc.x == 0.f || dc.y == 0.f;
         __syncthreads();  // every thread has read the DC term before it is overwritten
-        for (int ky = warp; ky <= ny / 2; ky += kGenWarps) {
+        const int at = s_lanes[lane];
+        for (int ky = warp * pl.rows + (at >> 10); ky <= ny / 2; ky += kGenWarps * pl.rows) {
             const int my = ky ? ny - ky : 0;
-            for (int kx = lane; kx < nx; kx += 32) {
+            for (int kx = at & 1023; kx < nx; kx += 32) {
                 const int mx = kx ? nx - kx : 0, t = ky * nx + kx, tm = my * nx + mx;
                 if (tm < t) continue;
                 const float2 A = plane[t], M = plane[tm];
@@ -479,9 +496,9 @@ __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel
         }
         int cnt = 0;
         if (g.Nps <= 4) {
-            cnt = gpeaks<4>(P, g.Nps, nx, ilo, ihi, jlo, jhi, pv, pi, parts);
+            cnt = gpeaks<4>(P, pl.rows, s_lanes, g.Nps, nx, ilo, ihi, jlo, jhi, pv, pi, parts);
         } else if (g.Nps <= 8) {
-            cnt = gpeaks<8>(P, g.Nps, nx, ilo, ihi, jlo, jhi, pv, pi, parts);
+            cnt = gpeaks<8>(P, pl.rows, s_lanes, g.Nps, nx, ilo, ihi, jlo, jhi, pv, pi, parts);
         } else {
             // Npeak_save rounds of a block arg-max over the local maxima
             float prev_v = FLT_MAX;
@@ -599,6 +616,7 @@ GenericPlan generic_plan(int wsx, int wsy)
     constants(wsx, pl.fx, pl.nfx, pl.mx, pl.px);
     constants(wsy, pl.fy, pl.nfy, pl.my, pl.py);
     pl.dx = div_magic32(wsx);
+    pl.rows = wsx < 32 ? 32 / wsx : 1;
     return pl;
 }
 
@@ -614,8 +632,10 @@ int xcorr_generic_ctas(int wsx, int wsy, int nps)
         if (sms <= 0) sms = 148;
     }
     if (xcorr_generic_needs_workspace(wsx, wsy)) return 2 * sms;
-    const size_t smem = table_bytes(wsx, wsy, nps) + (size_t)wsx * wsy * sizeof(float2);
-    const int by_smem = (int)((227 * 1024) / (smem + 1024));
+    // 228 KB an SM; a CTA also holds the kernel's own arrays and 1 KB of the system's
+    const size_t smem = table_bytes(wsx, wsy, nps) + (size_t)wsx * wsy * sizeof(float2) +
+                        kGenWarps * sizeof(PeakPart) + 32 * sizeof(uint16_t);
+    const int by_smem = (int)((228 * 1024) / (smem + 1024));
     const int per_sm = by_smem < 1 ? 1 : (by_smem > 8 ? 8 : by_smem);
     return per_sm * sms;
 }
