@@ -54,14 +54,9 @@ namespace {
 
 constexpr int kGenThreads = kGenericThreads;
 constexpr int kGenWarps = kGenThreads / 32;
-constexpr int kGenSmemPlane = 20480;  // complex points of a plane kept in shared memory
 
 // n / d by a multiply-high with ceil(2^32 / d) (0 for d = 1): exact while n * d < 2^32, and the
 // kernel's n stay below 2^20 points with d up to 1024.
-__host__ __device__ inline uint32_t div_magic32(int d)
-{
-    return d > 1 ? (uint32_t)((0x100000000ull + (uint64_t)d - 1) / (uint64_t)d) : 0u;
-}
 __device__ __forceinline__ int div_by(int n, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)n, magic) : n; }
 
 // a * w
@@ -571,11 +566,47 @@ __global__ void __launch_bounds__(kGenThreads, ANY ? 2 : 3) xcorr_generic_kernel
     }
 }
 
+// The launch of one instance.  ANY and SMEM have a module each (PIV_PART 2 * ANY + !SMEM), as the
+// driver loads a whole module with the first of its kernels: the first 40x40 pair of a process
+// waited 4.5 ms for one module of all, 1.6 for its own.
+template <bool ANY, bool SMEM>
+cudaError_t launch_generic(const XcorrArgs &a, const GenericPlan &pl, bool deformed, float2 *workspace, int ctas,
+                           size_t smem, cudaStream_t s)
+{
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto kern) {
+        // the largest any launch asks for: a captured launch of another grid's (larger) windows
+        // keeps running under the attribute set last
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+        if (e != cudaSuccess) return;
+        kern<<<ctas, kGenThreads, smem, s>>>(a, pl, workspace);
+        e = cudaGetLastError();
+    };
+    if (deformed) go(xcorr_generic_kernel<true, ANY, SMEM>);
+    else go(xcorr_generic_kernel<false, ANY, SMEM>);
+    return e;
+}
+#define PIV_GENERIC(ANY, SMEM) \
+    template cudaError_t launch_generic<ANY, SMEM>(const XcorrArgs &, const GenericPlan &, bool, float2 *, int, size_t, \
+                                                   cudaStream_t);
+
+#if PIV_PART
+PIV_GENERIC((PIV_PART >> 1) != 0, (PIV_PART & 1) == 0)
+#else
+extern PIV_GENERIC(false, false)
+extern PIV_GENERIC(true, true)
+extern PIV_GENERIC(true, false)
+
 // ---------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------
 
 namespace {
+constexpr int kGenSmemPlane = 20480;  // complex points of a plane kept in shared memory
+
+// the constant of div_by
+uint32_t div_magic32(int d) { return d > 1 ? (uint32_t)((0x100000000ull + (uint64_t)d - 1) / (uint64_t)d) : 0u; }
+
 int radices(int n, int *f)
 {
     int nf = 0;
@@ -651,28 +682,10 @@ cudaError_t launch_xcorr_generic(const XcorrArgs &a, bool deformed, float2 *work
                         (pl.in_smem ? (size_t)a.g.ws_x * a.g.ws_y * sizeof(float2) : 0);
     int ctas = pl.in_smem ? xcorr_generic_ctas(a.g.ws_x, a.g.ws_y, a.g.Nps) : workspace_ctas;
     if (ctas > n) ctas = n;
-    cudaError_t e = cudaSuccess;
-    auto go = [&](auto kern) {
-        // the largest any launch asks for: a captured launch of another grid's (larger) windows
-        // keeps running under the attribute set last
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-        if (e != cudaSuccess) return;
-        kern<<<ctas, kGenThreads, smem, s>>>(a, pl, workspace);
-        e = cudaGetLastError();
-    };
-    auto pick = [&](auto any, auto in_smem) {
-        constexpr bool A = decltype(any)::value, S = decltype(in_smem)::value;
-        if (deformed) go(xcorr_generic_kernel<true, A, S>);
-        else go(xcorr_generic_kernel<false, A, S>);
-    };
-    if (pl.any) {
-        if (pl.in_smem) pick(std::true_type{}, std::true_type{});
-        else pick(std::true_type{}, std::false_type{});
-    } else {
-        if (pl.in_smem) pick(std::false_type{}, std::true_type{});
-        else pick(std::false_type{}, std::false_type{});
-    }
-    return e;
+    const auto launch = pl.any ? (pl.in_smem ? launch_generic<true, true> : launch_generic<true, false>)
+                               : (pl.in_smem ? launch_generic<false, true> : launch_generic<false, false>);
+    return launch(a, pl, deformed, workspace, ctas, smem, s);
 }
+#endif
 
 }  // namespace piv
