@@ -663,9 +663,8 @@ __device__ __forceinline__ void merge_exchange_sort(float (&a)[N])
 // Median and MAD of one component of the 5x5 neighbourhood of (vx, vy) by a whole warp, slot q of
 // median_pass_kernel's network in lane q.  For NaN (candidates set by the caller) and medians that
 // are no number: what fminf and fmaxf make of those depends on the exchanges, so these are the
-// network's own.  About 100 instructions a neighbourhood; every lane gets the result.  Not inlined:
-// inlined, the 511 x 269 grid without NaN took 53 us instead of 51.
-__device__ __noinline__ float2 median5_warp(const float *src, const uint8_t *flag, int step, int Nx, int Ny, int vx,
+// network's own.  About 100 instructions a neighbourhood; every lane gets the result.
+__device__ __forceinline__ float2 median5_warp(const float *src, const uint8_t *flag, int step, int Nx, int Ny, int vx,
                                                int vy, int lane)
 {
     const unsigned all = 0xffffffffu;
@@ -695,6 +694,34 @@ __device__ __noinline__ float2 median5_warp(const float *src, const uint8_t *fla
     return make_float2(med, median());
 }
 
+// The components of a warp's neighbourhoods that need median5_warp, one after another: those with a
+// NaN, and those whose median is no number.  odd: this lane's neighbourhood holds an infinity or NaN.
+__device__ __noinline__ float2 median5_special(const float *px, const float *py, const uint8_t *flag, int step, int Nx,
+                                               int Ny, int v, bool odd, float med, float mad)
+{
+    const int lane = threadIdx.x & 31, vy = v / Nx, vx = v - vy * Nx;
+    bool special = odd && !(fabsf(med) < __int_as_float(0x7f800000));
+    if (odd && !special) {
+        const float *src = lane & 1 ? py : px;
+        for (int q = 0; q < 25 && !special; ++q) {
+            const int x = vx + q % 5 - 2, y = vy + q / 5 - 2;
+            if (q == 12 || x < 0 || x >= Nx || y < 0 || y >= Ny) continue;
+            const size_t id = (size_t)(y * Nx + x) * step;
+            special = flag[id] && src[id] != src[id];
+        }
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, special); todo; todo &= todo - 1) {
+        const int q = __ffs(todo) - 1;  // component q & 1, as this lane's by its own parity
+        const int qx = __shfl_sync(0xffffffffu, vx, q), qy = __shfl_sync(0xffffffffu, vy, q);
+        const float2 m = median5_warp(q & 1 ? py : px, flag, step, Nx, Ny, qx, qy, lane);
+        if (lane == q) {
+            med = m.x;
+            mad = m.y;
+        }
+    }
+    return make_float2(med, mad);
+}
+
 // The 5x5 stencil (the usual one): two threads per vector, one for each component, which meet by
 // shuffle for the decision.  A component's 24 neighbours are sorted by merge exchange (123
 // exchanges; the 32-slot bitonic network of median_pass_kernel has 240).  With all 24 present,
@@ -703,12 +730,12 @@ __device__ __noinline__ float2 median5_warp(const float *src, const uint8_t *fla
 // min(lower[i], upper[11 - i]).  What bounds it: the latency of the straight-line code on small
 // grids, issue slots on large ones.  Validation of a grid (two median passes, fill, smoothing), one
 // thread per vector with the general network -> this: 21 x 16 vectors 34 -> 23 us, 411 x 274
-// 64 -> 43 us, 384 x 509 98 -> 63 us.  Neighbourhoods that need the network's own exchanges
-// (median5_warp) are taken by the whole warp one after another: with 5 % of the candidates NaN
-// 511 x 269 vectors take 117 us (51 without; one thread per vector and the general network 91, a
-// thread's own loops over local memory 202), with infinities alone 57 to 75.  Other stencils keep
-// median_pass_kernel: the exchanges and
-// the two halves of the MAD are laid out for exactly 24 neighbours.
+// 64 -> 43 us, 384 x 509 98 -> 63 us.  Neighbourhoods with infinities or
+// NaN go through median5_special, out of line so that the others pay one vote for it: 511 x 269
+// vectors take 51 us without any, 67 to 86 with 1 to 20 % infinities, 87 and 113 with 1 and 5 % NaN
+// (one thread per vector and the general network 84 to 104; a thread's own loops over local memory
+// 166 to 212).  Other stencils keep median_pass_kernel: the exchanges and the two halves of the MAD
+// are laid out for exactly 24 neighbours.
 __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
 {
     chain_start();
@@ -723,7 +750,7 @@ __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
     const float inf = __int_as_float(0x7f800000);
     float s[24];
     int n = 0;
-    bool odd = false;  // a NaN
+    bool odd = false;  // an infinity or a NaN
 #pragma unroll
     for (int q = 0; q < 25; ++q) {
         if (q == 12) continue;  // the centre
@@ -734,7 +761,7 @@ __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
         const float f = src[id];
         s[q < 12 ? q : q - 1] = ok ? f : inf;
         n += ok;
-        odd |= ok && f != f;
+        odd |= ok && !(fabsf(f) < inf);
     }
     merge_exchange_sort<24, 16>(s);
     float med, mad;
@@ -760,21 +787,15 @@ __global__ void __launch_bounds__(128) median5_pass_kernel(const MedianPass a)
         bitonic_step<32, 32, 16>(w);
         mad = median_sorted<32>(w, n);
     }
-    const bool judged = n >= a.minN && n >= 1;
-    for (unsigned todo = __ballot_sync(0xffffffffu, judged && (odd || !(fabsf(med) < inf))); todo; todo &= todo - 1) {
-        const int q = __ffs(todo) - 1;  // component q & 1, as this lane's by its own parity
-        const int qx = __shfl_sync(0xffffffffu, vx, q), qy = __shfl_sync(0xffffffffu, vy, q);
-        const float *from = a.ix ? (q & 1 ? a.iy : a.ix) : (q & 1 ? a.cdy : a.cdx);
-        const float2 m = median5_warp(from, flag, step, a.Nx, a.Ny, qx, qy, threadIdx.x & 31);
-        if ((threadIdx.x & 31) == q) {
-            med = m.x;
-            mad = m.y;
-        }
+    if (__any_sync(0xffffffffu, odd)) {
+        const float2 m = median5_special(a.ix ? a.ix : a.cdx, a.ix ? a.iy : a.cdy, flag, step, a.Nx, a.Ny, v, odd, med, mad);
+        med = m.x;
+        mad = m.y;
     }
     // median_filtering's decision (median_decide): the first valid candidate with both residuals
     // below the threshold
     const float epsilon = 0.1f;
-    bool found = !judged, ok = false;
+    bool found = !(n >= a.minN && n >= 1), ok = false;
     float r = 0.f;
     for (int i = 0; i < a.Nps; ++i) {
         const size_t c = (size_t)v * a.Nps + i;
