@@ -661,9 +661,8 @@ int tune_xcorr(piv_engine *e)
     cudaStream_t s = e->stream;
     CK(launch_pattern(e->d_f1, nullptr, e->pitch, e->pitch, e->rows, 1u, s));
     CK(launch_pattern(e->d_f2, nullptr, e->pitch, e->pitch, e->rows, 2u, s));
-    cudaEvent_t a, b;
-    CK(cudaEventCreate(&a));
-    CK(cudaEventCreate(&b));
+    cudaEvent_t ev[9];
+    for (cudaEvent_t &v : ev) CK(cudaEventCreate(&v));
     int rc = PIV_OK;
     for (int k = 0; k < 2 && !rc; ++k) {
         GridState &gs = e->grid[k];
@@ -672,28 +671,28 @@ int tune_xcorr(piv_engine *e)
         if (nv <= 1) continue;
         const bool deformed = gs.def != nullptr;
         if (deformed) CK(launch_pattern(nullptr, gs.def, gs.def_pitch, gs.gg.Nx_aug, gs.gg.Ny_aug, 3u + k, s));
-        float best = 1e30f;
-        int best_v = 0;
-        for (int v = 0; v < nv && v < 8 && !rc; ++v) {
-            gs.variant = v;
-            if ((rc = do_xcorr(e, k, deformed, 0, 0, nullptr))) break;  // warm-up
-            cudaEventRecord(a, s);
-            for (int r = 0; r < 2 && !rc; ++r) rc = do_xcorr(e, k, deformed, 0, 0, nullptr);
-            cudaEventRecord(b, s);
-            if (cudaEventSynchronize(b) != cudaSuccess) {
-                rc = set_err(e, PIV_ERR_CUDA, "autotune timing failed");
-                break;
+        // one launch of each variant in turn, three times over (the first to warm up): a launch then
+        // finds another kernel's code in the instruction caches, as it does in a pair
+        const int tried = nv < 8 ? nv : 8;
+        std::fill_n(gs.tuned_ms, tried, 0.f);
+        for (int round = 0; round < 3 && !rc; ++round) {
+            cudaEventRecord(ev[0], s);
+            for (int v = 0; v < tried && !rc; ++v) {
+                gs.variant = v;
+                rc = do_xcorr(e, k, deformed, 0, 0, nullptr);
+                cudaEventRecord(ev[v + 1], s);
             }
-            float ms = 0;
-            cudaEventElapsedTime(&ms, a, b);
-            gs.tuned_ms[v] = ms / 2;
-            if (ms < best) {
-                best = ms;
-                best_v = v;
+            if (!rc && cudaEventSynchronize(ev[tried]) != cudaSuccess)
+                rc = set_err(e, PIV_ERR_CUDA, "autotune timing failed");
+            for (int v = 0; v < tried && !rc && round > 0; ++v) {
+                float ms = 0;
+                cudaEventElapsedTime(&ms, ev[v], ev[v + 1]);
+                gs.tuned_ms[v] += 0.5f * ms;
             }
         }
+        const int best_v = (int)(std::min_element(gs.tuned_ms, gs.tuned_ms + tried) - gs.tuned_ms);
         gs.variant = best_v;
-        gs.n_tuned = nv < 8 ? nv : 8;
+        gs.n_tuned = tried;
         // leave no trace of the tuning input
         if (deformed) CK(cudaMemsetAsync(gs.def, 0, (size_t)gs.def_pitch * gs.gg.Ny_aug * sizeof(float), s));
         const size_t Nt = (size_t)gs.gg.Nt_vec, Nc = Nt * p.Npeak_save;
@@ -704,8 +703,7 @@ int tune_xcorr(piv_engine *e)
         CK(cudaMemsetAsync(gs.pidx, 0xff, Nc * sizeof(int), s));
         CK(cudaMemsetAsync(gs.pval, 0, Nc * sizeof(float), s));
     }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    for (cudaEvent_t v : ev) cudaEventDestroy(v);
     CK(cudaMemsetAsync(e->d_f1, 0, (size_t)e->pitch * e->rows, s));
     CK(cudaMemsetAsync(e->d_f2, 0, (size_t)e->pitch * e->rows, s));
     CK(cudaStreamSynchronize(s));
