@@ -421,7 +421,7 @@ def run_ours(args, rank, world, local):
     achieved = flops / (kms * 1e-3) / 1e12
     roofline = {"bound": "fp32", "achieved": round(achieved, 2), "peak": round(peak, 2), "unit": "TFLOP/s",
                 "frac": round(achieved / peak, 4), "traffic": traffic_from_profile(),
-                "kernel": "xcorr_peak_kernel<32,32> (grid-2 correlation, deformed)",
+                "kernel": "grid-2 correlation of 32x32 windows, deformed (the tuned variant; xcorr_pair_kernel at this size)",
                 "kernel_ms": round(kms, 4), "algorithmic_flops_per_launch": flops,
                 "peak_source": "FP32 FMA peak measured live on this GPU by piv_probe_fp32_peak"}
     launches = e.launches_per_pair() * args.steps

@@ -489,11 +489,7 @@ struct MedianPass {
     int *zero_n;         // set to 0 by a pass before the one that appends
 };
 
-// One pass of organize_median_filter_data + median_validity + Calc_median x4 +
-// Calc_devi x2 + median_filtering (X/xcorr2d_multi_grid.cu:209-296, 1464-1513), one
-// thread per vector.  Neighbours are gathered in raster stencil order with the centre
-// slot (wx*wy-1)/2 skipped; the medians are order statistics, so the gather order
-// does not change them.
+// Neighbours are gathered in raster stencil order with the centre slot (wx*wy-1)/2 skipped.
 __device__ __forceinline__ void median_neighbour(const MedianPass &a, int id, bool &ok, float &fxv, float &fyv)
 {
     if (a.ix) {
@@ -534,41 +530,41 @@ __device__ __forceinline__ void median_vector32(const MedianPass &a, int v, floa
     const int Ntm = a.wx * a.wy, centre = (Ntm - 1) / 2;
     const int vy = v / a.Nx, vx = v - vy * a.Nx;
     const int hfwx = (a.wx - 1) / 2, hfwy = (a.wy - 1) / 2;
-                const float inf = __int_as_float(0x7f800000);
-                float xs[32], ys[32];
-                int n = 0;
-                int tx = 0, ty = 0;  // stencil column and row of slot t (no division per slot)
-    #pragma unroll
-                for (int t = 0; t < 32; ++t) {
-                    const int x = vx - hfwx + tx, y = vy - hfwy + ty;
-                    const bool inb = (t < Ntm) & (t != centre) & (x >= 0) & (x <= a.Nx - 1) & (y >= 0) & (y <= a.Ny - 1);
-                    bool ok;
-                    float px, py;
-                    median_neighbour(a, inb ? y * a.Nx + x : v, ok, px, py);  // always a valid address
-                    ok = ok & inb;
-                    xs[t] = ok ? px : inf;
-                    ys[t] = ok ? py : inf;
-                    n += ok;
-                    const bool wrap = ++tx == a.wx;
-                    tx = wrap ? 0 : tx;
-                    ty += wrap;
-                }
-                if (n >= a.minN && n >= 1) {
-                    bitonic_sort<32>(xs);
-                    bitonic_sort<32>(ys);
-                    const float mx = median_sorted<32>(xs, n), my = median_sorted<32>(ys, n);
-                    // |x - median| over a sorted x falls, then rises (then +inf): a bitonic
-                    // sequence, which the final merge stage of the network sorts on its own
-    #pragma unroll
-                    for (int q = 0; q < 32; ++q) {
-                        xs[q] = (q < n) ? fabsf(xs[q] - mx) : inf;
-                        ys[q] = (q < n) ? fabsf(ys[q] - my) : inf;
-                    }
-                    bitonic_step<32, 32, 16>(xs);
-                    bitonic_step<32, 32, 16>(ys);
-                    const float dmx = median_sorted<32>(xs, n), dmy = median_sorted<32>(ys, n);
-                    median_decide(a, v, mx, my, dmx, dmy, rx, ry, rv);
-                }
+    const float inf = __int_as_float(0x7f800000);
+    float xs[32], ys[32];
+    int n = 0;
+    int tx = 0, ty = 0;  // stencil column and row of slot t (no division per slot)
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+        const int x = vx - hfwx + tx, y = vy - hfwy + ty;
+        const bool inb = (t < Ntm) & (t != centre) & (x >= 0) & (x <= a.Nx - 1) & (y >= 0) & (y <= a.Ny - 1);
+        bool ok;
+        float px, py;
+        median_neighbour(a, inb ? y * a.Nx + x : v, ok, px, py);  // always a valid address
+        ok = ok & inb;
+        xs[t] = ok ? px : inf;
+        ys[t] = ok ? py : inf;
+        n += ok;
+        const bool wrap = ++tx == a.wx;
+        tx = wrap ? 0 : tx;
+        ty += wrap;
+    }
+    if (n >= a.minN && n >= 1) {
+        bitonic_sort<32>(xs);
+        bitonic_sort<32>(ys);
+        const float mx = median_sorted<32>(xs, n), my = median_sorted<32>(ys, n);
+        // |x - median| over a sorted x falls, then rises (then +inf): a bitonic
+        // sequence, which the final merge stage of the network sorts on its own
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            xs[q] = (q < n) ? fabsf(xs[q] - mx) : inf;
+            ys[q] = (q < n) ? fabsf(ys[q] - my) : inf;
+        }
+        bitonic_step<32, 32, 16>(xs);
+        bitonic_step<32, 32, 16>(ys);
+        const float dmx = median_sorted<32>(xs, n), dmy = median_sorted<32>(ys, n);
+        median_decide(a, v, mx, my, dmx, dmy, rx, ry, rv);
+    }
 }
 
 // One pass of organize_median_filter_data + median_validity + Calc_median x4 +

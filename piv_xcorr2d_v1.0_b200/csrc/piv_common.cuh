@@ -22,9 +22,10 @@ namespace piv {
 // loads: the read-only path (__ldg) is for data that nothing writes while the kernel is resident.
 // The correlation kernels call chain_start() for the kernel after them, but are launched in the
 // ordinary way: they want most of an SM's shared memory, and setting them up beside a running
-// kernel costs more than it saves (a pair of 333x251: 112 us this way, 125 with all chained, 113 to
-// 117 with none; 1024x1024: 235, 236, 238).  Kernels launched from the host one after another, as
-// the stand-alone enhancement, gain most: 27.6 -> 23.4 us for a 4096x2160 frame.
+// kernel costs more than it saves (a pair of 333x251 took 112 us this way, 125 with all chained).
+// Chained against none, a call through the public API: 333x251 128 us, 138; 1024x1024 255, 260;
+// 2048x1536 with 16 px windows and 6600x4400 the same.  Kernels launched from the host one after
+// another, as the stand-alone enhancement, gain most: a 4096x2160 frame 20.6 us, 24.6.
 __device__ __forceinline__ void chain_start()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -1,7 +1,10 @@
 // xcorr_dispatch.cu -- window shape and variant -> instantiated fused correlation kernel.
 // Every shape (WSX, WSY) is compiled in translation units of its own (xcorr_shape_*.cu) in
 // several variants (B windows per CTA, NT threads per CTA); the first listed variant of a
-// shape is its default, the engine's autotuner may pick another one per grid.
+// shape is its default, the engine's autotuner may pick another one per grid.  No size decides which
+// is the fastest: small CTAs win while the grid is about one wave, as their windows are done sooner,
+// and the more economical forms above.  32x32: 300 windows (333x251) 9.9 us a launch with 4 windows
+// per CTA, 11.4 by the warp form; 744 (512x384) 10.5 and 12.3; 3,969 (1024x1024) 21.7 and 19.5.
 #include <cstring>
 #include <type_traits>
 

@@ -634,11 +634,10 @@ __device__ __forceinline__ void peak_window_merge(const XcorrArgs &a, const floa
 
 // Residency asked of the register allocation (the second __launch_bounds__ argument), where
 // the compiler's own choice leaves the SM's shared memory unused: 64x64 with 2 windows per CTA
-// of 128 threads (68 KB: 3 CTAs at 168 registers and 160 bytes of spills, 0.547 ms a grid-1
-// launch at 6600x4400; unbounded 217 registers and 2 CTAs, 0.685), 32x64 with 4 windows per 128
-// threads or 2 per 64 (12 warps at 168 registers and 224 to 256 bytes of spills; a launch at
-// 4096x2160 and spacing 8x16 668 and 692 us, unbounded at 213 registers 726 and 712, 1024x768
-// and spacing 16x32 19.3 and 20.8 us against 24.1 and 23.7), 32x32 with 4 windows per CTA of 128
+// of 128 threads (68 KB: 3 CTAs at 168 registers, 0.551 ms a grid-1 launch at 6600x4400; unbounded
+// 217 registers and 2 CTAs, 0.685), 32x64 with 4 windows per 128 threads or 2 per 64 (12 warps at
+// 168 registers; a launch at 4096x2160 and spacing 8x16 668 and 692 us, unbounded at 213 registers
+// 726 and 712, 1024x768 and spacing 16x32 19.3 and 20.8 us against 24.1 and 23.7), 32x32 with 4 windows per CTA of 128
 // threads (5 CTAs at 96 registers).
 template <int WSX, int WSY, int B, int NT>
 constexpr int xcorr_min_ctas()
@@ -690,8 +689,8 @@ __device__ __forceinline__ int batch_pair(const XcorrBatch &b, int it)
 // half in shared memory, which lets 16 warps share an SM (12.6 KB of shared memory and 128
 // registers a thread each; the CTA form's 16.9 KB a pair allow 12).  113,300 windows of the
 // 6600x4400 grid 2 take 0.344 ms; the best CTA form (8 windows, 128 threads) 0.407 ms, and
-// 0.464 ms before packed transforms and staged loads.  What bounds it: issue slots (2,240 warp
-// instructions per window, 60 % of the slots used), then the latency of 16 warps.
+// 0.464 ms before packed transforms and staged loads.  What bounds it: issue slots (2,310 warp
+// instructions per window, 59 % of the slots used), then latency: 14 of 16 possible warps active.
 template <int K>
 struct PairShared {
     using L = Plane<32, 32>;
